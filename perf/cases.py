@@ -1,0 +1,514 @@
+"""Measured cases of the library: steps of ``Engine.step``, the one entry point that prompts and decoded tokens go
+through, on the configurations that the benchmark and the tests use (random weights).
+
+A case is one step of one engine. ``step`` "decode": ``batch`` sequences that hold between ``low`` and ``high`` cached
+positions bring one token each. ``step`` "prompt": ``batch`` sequences bring between ``low`` and ``high`` new tokens on
+top of ``cached`` positions; the logits of each sequence's last ``want`` tokens are wanted (0: of every token). The
+architectures are the dense Llama-arch decoder (the library's main one; its 3B-shaped sizes are the benchmark's), the
+decoder with a mixture of experts (Vozinex) and the hybrid of windowed, latent and linear attention (Nilatar), each at
+sizes of its benchmark.
+"""
+from __future__ import annotations
+
+import math
+import zlib
+
+import torch
+
+PAGE = 64                    # positions of a cache page
+
+# layer sizes of the benchmark's configurations
+LLAMA_3B = dict(arch="llama", width=2560, heads=20, kv=4, dim=128, ff=10496, theta=70000000.0, eps=1e-5)
+LLAMA_16B = dict(LLAMA_3B, width=5120, heads=40, kv=8, ff=13824)
+# a decoder of the smallest sizes that the serving kernels are used at (heads of 64)
+LLAMA_SMALL = dict(arch="llama", width=512, heads=8, kv=2, dim=64, ff=1408, theta=10000.0, eps=1e-5)
+LLAMA_1K = dict(arch="llama", width=1024, heads=8, kv=2, dim=128, ff=2816, theta=10000.0, eps=1e-5)
+VOZINEX = {"s": dict(width=1024, heads=8, kv=2, experts=16, top=4, ff=512),
+           "m": dict(width=2048, heads=16, kv=4, experts=32, top=4, ff=1024),
+           "l": dict(width=4096, heads=32, kv=8, experts=32, top=4, ff=2048)}
+VOZINEX_WINDOW, VOZINEX_KEEP = 1024, 4
+NILATAR = {"s": dict(width=1024, heads=8, kv=2, ff=2816, q_rank=384, lat=64),
+           "m": dict(width=2048, heads=16, kv=4, ff=5632, q_rank=768, lat=64),
+           "l": dict(width=4096, heads=32, kv=8, ff=11008, q_rank=1536, lat=128)}
+NILATAR_WINDOW, NILATAR_KV_RANK, NILATAR_ROT = 1024, 96, 32
+
+
+def _case(name, sizes, **more):
+    c = dict(sizes, dtype="bfloat16", vocab=32768, cached=0, want=1)
+    c.update(more)
+    if name:
+        c["name"] = name
+    return c
+
+
+def _vozinex(size):
+    return dict(VOZINEX[size], arch="vozinex", dim=128, theta=10000.0, eps=1e-5)
+
+
+def _nilatar(size):
+    return dict(NILATAR[size], arch="nilatar", dim=128, theta=10000.0, eps=1e-5)
+
+
+def listed():
+    return [
+        # one user's chat: a whole 3B-shaped model decodes one sequence, a short context (latency of a token)
+        _case("decode_3b_one", LLAMA_3B, layers=32, vocab=166144, step="decode", batch=1, low=517, high=517),
+        # the benchmark's own workload: eight sequences at a context of 8192
+        _case("decode_3b_eight", LLAMA_3B, layers=32, vocab=166144, step="decode", batch=8, low=8191, high=8191),
+        # a busy server: many sequences of very unequal lengths (eight of the layers)
+        _case("decode_3b_many", LLAMA_3B, layers=8, step="decode", batch=48, low=203, high=6007),
+        # the smallest model and step: launches and latency are all there is
+        _case("decode_small", LLAMA_SMALL, layers=4, vocab=4096, step="decode", batch=1, low=100, high=100),
+        # the benchmark's prompt: 2048 tokens (eight of the layers)
+        _case("prompt_3b_2048", LLAMA_3B, layers=8, vocab=166144, step="prompt", batch=1, low=2048, high=2048),
+        # short chat turns that start together, of odd lengths
+        _case("prompt_3b_short", LLAMA_3B, layers=8, step="prompt", batch=3, low=37, high=181),
+        # further turns of two long conversations: new tokens on top of cached ones, the last of them drafts to be checked
+        _case("prompt_3b_further", LLAMA_3B, layers=8, step="prompt", batch=2, low=391, high=823, cached=4011, want=9),
+        # a long document through layers of the 16B-shaped configuration, near the longest single step
+        _case("prompt_16b_long", LLAMA_16B, layers=2, step="prompt", batch=1, low=8171, high=8171),
+        # mixture of experts: decoded tokens behind a window, and a prompt whose tokens are scored
+        _case("decode_experts", _vozinex("m"), layers=4, step="decode", batch=8, low=1500, high=4000),
+        _case("prompt_experts", _vozinex("m"), layers=2, step="prompt", batch=1, low=2048, high=2048, want=100),
+        # the hybrid decoder's three mixers over an odd prompt
+        _case("prompt_hybrid", _nilatar("m"), layers=4, step="prompt", batch=1, low=1777, high=1777),
+        # the true 32-bit path, as a check of a model's numbers runs it
+        _case("prompt_float32", LLAMA_1K, layers=4, step="prompt", batch=2, low=201, high=313, dtype="float32",
+              want=0),
+    ]
+
+
+def _log_int(rng, low, high):
+    return int(round(math.exp(rng.uniform(math.log(low), math.log(high)))))
+
+
+def draw(rng):
+    kind = rng.choice(["decode", "decode", "decode", "prompt", "prompt", "prompt", "experts_decode", "experts_prompt",
+                       "hybrid_prompt", "float32"])
+    if kind in ("decode", "prompt"):
+        sizes = dict(rng.choice([LLAMA_SMALL, LLAMA_1K, LLAMA_3B, LLAMA_3B, LLAMA_16B]))
+        sizes["ff"] = max(16, int(sizes["ff"] * rng.uniform(0.6, 1.2)) // 16 * 16)
+    if kind == "decode":
+        batch = _log_int(rng, 1, 64)
+        high = _log_int(rng, 33, min(16384, 200000 // batch))
+        return _case("", sizes, layers=rng.randint(4, 8), step="decode", batch=batch,
+                     low=max(16, int(high * rng.uniform(0.1, 1.0))), high=high)
+    if kind == "prompt":
+        batch = rng.randint(1, 4)
+        high = _log_int(rng, 17, 6000 // batch)
+        return _case("", sizes, layers=rng.randint(2, 4), step="prompt", batch=batch,
+                     low=max(9, int(high * rng.uniform(0.3, 1.0))), high=high, cached=rng.choice([0, 0, rng.randint(1, 3000)]),
+                     want=rng.choice([1, 1, 5]))
+    if kind == "experts_decode":
+        high = _log_int(rng, 100, 6000)
+        return _case("", _vozinex(rng.choice("sml")), layers=rng.randint(2, 4), step="decode", batch=_log_int(rng, 1, 40),
+                     low=max(33, high // rng.randint(1, 6)), high=high)
+    if kind == "experts_prompt":
+        high = _log_int(rng, 33, 2400)
+        return _case("", _vozinex(rng.choice("sm")), layers=2, step="prompt", batch=rng.randint(1, 2), low=max(17, high // 2),
+                     high=high, want=rng.choice([1, 17]))
+    if kind == "hybrid_prompt":
+        high = _log_int(rng, 65, 2400)
+        return _case("", _nilatar(rng.choice("sm")), layers=4, step="prompt", batch=rng.randint(1, 2), low=max(33, high // 2),
+                     high=high, want=rng.choice([1, 30]))
+    high = _log_int(rng, 17, 400)
+    step = rng.choice(["decode", "prompt"])
+    return _case("", LLAMA_1K, layers=rng.randint(2, 4), step=step, batch=rng.randint(1, 3), low=max(9, high // 2), high=high,
+                 dtype="float32", want=rng.choice([0, 1]))
+
+
+# ---------------------------------------------------------------------------------------------- the case's numbers
+def _lengths(case):
+    """each sequence's cached length (decode) or number of new tokens (prompt): from ``low`` to ``high``, unevenly"""
+    n, low, high = case["batch"], case["low"], case["high"]
+    out = [high - (high - low) * (i * 5 % n) // max(1, n - 1) for i in range(n)] if n > 1 else [high]
+    if case["step"] == "decode" and case["arch"] == "vozinex":
+        # (the sequence goes back by one position after the step: the oldest position in its window must not be the last
+        # of a page, which the cache gives back when the window has passed it)
+        out = [m + 1 if (m + 2 - VOZINEX_WINDOW) % PAGE == 0 else m for m in out]
+    return out
+
+
+def _tokens(case, seed):
+    g = torch.Generator().manual_seed(seed * 7919 + 11)
+    counts = [1] * case["batch"] if case["step"] == "decode" else _lengths(case)
+    return [tuple(torch.randint(0, case["vocab"], (n,), generator=g).tolist()) for n in counts]
+
+
+def _want(case, n):
+    """the places among a sequence's n tokens whose logits are wanted"""
+    return tuple(range(max(0, n - case["want"]) if case["want"] else 0, n))
+
+
+def _cached(case):
+    return _lengths(case) if case["step"] == "decode" else [case["cached"]] * case["batch"]
+
+
+def _config(case):
+    """the model's config.json object"""
+    c = case
+    if c["arch"] == "llama":
+        return dict(architectures=["LlamaForCausalLM"], model_type="llama", vocab_size=c["vocab"], hidden_size=c["width"],
+                    intermediate_size=c["ff"], num_hidden_layers=c["layers"], num_attention_heads=c["heads"],
+                    num_key_value_heads=c["kv"], head_dim=c["dim"], rms_norm_eps=c["eps"], rope_theta=c["theta"],
+                    tie_word_embeddings=False)
+    if c["arch"] == "vozinex":
+        mixer = {"heads": c["heads"], "kv_heads": c["kv"], "dim": c["dim"], "vdim": c["dim"], "scale": c["dim"] ** -0.5,
+                 "rot": {"base": c["theta"], "dims": c["dim"] // 2},
+                 "mask": {"size": VOZINEX_WINDOW, "keep_first": VOZINEX_KEEP}}
+        mlp = {"kind": "moe", "expert": {"ff": c["ff"]}, "router": {"experts": c["experts"], "top": c["top"]}}
+        return {"architecture": "Vozinex", "vocab": c["vocab"], "width": c["width"], "norm": {"eps": c["eps"]},
+                "layers": [{"type": "attention", "mixer": mixer, "mlp": mlp} for _ in range(c["layers"])],
+                "loop": {"start": 0, "stop": 0, "times": 1}}
+    att, lat, lin = _nilatar_mixers(c)
+    ff = {"kind": "dense", "ff": c["ff"]}
+    return {"architecture": "Nilatar", "vocab": c["vocab"], "width": c["width"], "norm": {"eps": c["eps"]},
+            "embedding": {"scale": 1.0},
+            "layers": [{"type": "attention", "mixer": att, "mlp": ff}, {"type": "latent_attention", "mixer": lat, "mlp": ff},
+                       {"type": "lightning", "mixer": lin, "mlp": ff},
+                       {"type": "attention", "mixer": dict(att, kv_from=0), "mlp": ff}]}
+
+
+def _nilatar_mixers(c):
+    h, d, lat, r = c["heads"], c["dim"], c["lat"], NILATAR_ROT
+    att = {"heads": h, "kv_heads": c["kv"], "dim": d, "vdim": d, "scale": d ** -0.5, "mask": {"size": NILATAR_WINDOW}}
+    latent = {"heads": h, "dim": lat, "rot_dim": r, "vdim": lat, "q_rank": c["q_rank"], "kv_rank": NILATAR_KV_RANK,
+              "scale": (lat + r) ** -0.5,
+              "rot": {"base": c["theta"], "dims": r, "scaling": {"factor": 8.0, "original": 4096, "fast": 16.0, "slow": 2.0}}}
+    lin = {"heads": h, "dim": d, "vdim": d, "decay": [1.0 - 2.0 ** (-5.0 - 3.0 * i / max(1, h - 1)) for i in range(h)]}
+    return att, latent, lin
+
+
+def _shapes(case):
+    """{tensor name: shape} of the model"""
+    c, out = case, {}
+    e, q, kv = c["width"], c["heads"] * c["dim"], c["kv"] * c["dim"]
+    if c["arch"] == "llama":
+        out["model.embed_tokens.weight"] = (c["vocab"], e)
+        for i in range(c["layers"]):
+            p = "model.layers.%d." % i
+            out.update({p + "input_layernorm.weight": (e,), p + "self_attn.q_proj.weight": (q, e),
+                        p + "self_attn.k_proj.weight": (kv, e), p + "self_attn.v_proj.weight": (kv, e),
+                        p + "self_attn.o_proj.weight": (e, q), p + "post_attention_layernorm.weight": (e,),
+                        p + "mlp.gate_proj.weight": (c["ff"], e), p + "mlp.up_proj.weight": (c["ff"], e),
+                        p + "mlp.down_proj.weight": (e, c["ff"])})
+        out.update({"model.norm.weight": (e,), "lm_head.weight": (c["vocab"], e)})
+        return out
+    out["embed"] = (c["vocab"], e)
+    for i in range(c["layers"]):
+        p, m = "l%d." % i, "l%d.mix." % i
+        out.update({p + "norm1": (e,), p + "norm2": (e,)})
+        if c["arch"] == "vozinex":
+            out.update({p + "norm1.b": (e,), p + "norm2.b": (e,), m + "q": (q, e), m + "k": (kv, e), m + "v": (kv, e),
+                        m + "o": (e, q), m + "q.norm": (q,), m + "k.norm": (kv,), p + "mlp.router": (c["experts"], e),
+                        p + "mlp.router.b": (c["experts"],)})
+            for j in range(c["experts"]):
+                out.update({p + "mlp.e%d.up" % j: (c["ff"], e), p + "mlp.e%d.down" % j: (e, c["ff"])})
+            continue
+        out.update({p + "ls1": (e,), p + "ls2": (e,), p + "mlp.gate": (c["ff"], e), p + "mlp.up": (c["ff"], e),
+                    p + "mlp.down": (e, c["ff"])})
+        if i == 1:
+            h, d, r, kr = c["heads"], c["lat"], NILATAR_ROT, NILATAR_KV_RANK
+            out.update({m + "dq": (c["q_rank"], e), m + "dq.norm": (c["q_rank"],), m + "uq": (h * (d + r), c["q_rank"]),
+                        m + "dkv": (kr + r, e), m + "dkv.norm": (kr,), m + "uk": (h * d, kr), m + "uv": (h * d, kr),
+                        m + "g": (h * d, e), m + "o": (e, h * d)})
+        elif i == 2:
+            out.update({m + x: (q, e) for x in "qkvg"})
+            out.update({m + "norm": (q,), m + "o": (e, q)})
+        else:
+            out.update({m + "q": (q, e), m + "g": (q, e), m + "o": (e, q), m + "sink": (c["heads"],)})
+            if i == 0:
+                out.update({m + "k": (kv, e), m + "v": (kv, e)})
+    out["final.norm"] = (e,)
+    if c["arch"] == "vozinex":
+        out["final.norm.b"] = (e,)
+    out["head"] = (c["vocab"], e)
+    return out
+
+
+def _generator(seed, name):
+    return torch.Generator(device="cuda").manual_seed((seed << 32) + zlib.crc32(name.encode()))
+
+
+def _tensor(case, name, shape, seed):
+    """a weight as the model folder holds it: gains around one, biases of zero, everything else N(0, 0.02)"""
+    if name.endswith(".b"):
+        return torch.zeros(shape, dtype=torch.float32, device="cuda").to(getattr(torch, case["dtype"]))
+    t = torch.empty(shape, dtype=torch.float32, device="cuda").normal_(0.0, 0.02, generator=_generator(seed, name))
+    if len(shape) == 1 and not name.endswith("sink"):
+        t += 1.0
+    return t.to(getattr(torch, case["dtype"]))
+
+
+def _history(case, layer, b, n, seed):
+    """the keys and values [pages, 2, kv, 64, dim] that sequence b's cached positions hold in a layer: N(0, 1)"""
+    t = torch.empty(-(-n // PAGE), 2, case["kv"], PAGE, case["dim"], dtype=getattr(torch, case["dtype"]), device="cuda")
+    return t.normal_(0.0, 1.0, generator=_generator(seed, "history.%d.%d" % (layer, b)))
+
+
+# ---------------------------------------------------------------------------------------------- a user's program
+def prepare(case, seed):
+    from kindi_b200.config import model_from_config
+    from kindi_b200.engine.batch import StepEntry
+    from kindi_b200.engine.engine import Engine
+    _, spec = model_from_config(_config(case))
+    tokens, cached = _tokens(case, seed), _cached(case)
+    totals = [n + len(t) for n, t in zip(cached, tokens)]
+    eng = Engine(spec=spec, tensors={n: _tensor(case, n, s, seed) for n, s in _shapes(case).items()}, dtype=case["dtype"],
+                 ctx=sum(-(-n // PAGE) * PAGE for n in totals) + PAGE, max_batch=case["batch"])
+    state = {"engine": eng, "tokens": tokens, "cached": cached, "slots": None, "want": [_want(case, len(t)) for t in tokens]}
+    if any(cached):
+        # sequences that earlier steps left in the cache
+        state["slots"] = [eng.alloc() for _ in cached]
+        for b, (slot, n) in enumerate(zip(state["slots"], cached)):
+            eng.cache.reserve(slot, n)
+            eng.cache.flush()
+            for layer in range(case["layers"]):
+                pool, table, _ = eng.cache.kv_view(layer)
+                pool[table[slot, :-(-n // PAGE)].long()] = _history(case, layer, b, n, seed)
+            eng.cache.commit(slot, n)
+    if state["slots"] is not None:
+        state["entries"] = [StepEntry(s, t, w) for s, t, w in zip(state["slots"], tokens, state["want"])]
+    for _ in range(2):                     # a server's engine has seen the step's shape before: it is recorded by now
+        run(state)
+    torch.cuda.synchronize()
+    return state
+
+
+def run(state):
+    from kindi_b200.engine.batch import StepEntry
+    eng = state["engine"]
+    if state["slots"] is None:
+        # whole prompts: a request arrives, its prompt runs, and it leaves
+        slots = [eng.alloc() for _ in state["tokens"]]
+        logits = eng.step([StepEntry(s, t, w) for s, t, w in zip(slots, state["tokens"], state["want"])])
+        for s in slots:
+            eng.free(s)
+        return logits
+    logits = eng.step(state["entries"])
+    # the sequences go back to their cached length, as when a drafted token is dropped or a turn is sent again
+    for slot, n in zip(state["slots"], state["cached"]):
+        eng.cache.commit(slot, n)
+    return logits
+
+
+# ---------------------------------------------------------------------------------------------- what a step cannot do without
+def work(case):
+    c = case
+    el = 4 if c["dtype"] == "float32" else 2
+    counts = [1] * c["batch"] if c["step"] == "decode" else _lengths(c)
+    rows, cached, wanted = sum(counts), _cached(c), sum(len(_want(c, n)) for n in counts)
+    matrices = head = 0
+    for name, s in _shapes(c).items():
+        if name in ("model.embed_tokens.weight", "embed") or len(s) == 1:
+            continue
+        if name in ("lm_head.weight", "head"):
+            head = s[0] * s[1]
+        elif ".mlp.e" not in name:
+            matrices += s[0] * s[1]
+    bytes_, flops = (matrices + head) * el, 2.0 * matrices * rows + 2.0 * head * wanted
+    if c["arch"] == "vozinex":
+        one, picks = 2 * c["width"] * c["ff"], rows * c["top"]
+        touched = c["experts"] * (1.0 - (1.0 - c["top"] / c["experts"]) ** rows)
+        bytes_ += c["layers"] * touched * one * el
+        flops += c["layers"] * 2.0 * picks * one
+    # keys and values: each cached position read once, each new one written; scores and sums over the visible pairs
+    window = {"vozinex": VOZINEX_WINDOW, "nilatar": NILATAR_WINDOW}.get(c["arch"])
+    read = pairs = full_pairs = 0
+    for n, m in zip(cached, counts):
+        seen = n if window is None else min(n, window)
+        read += seen
+        full_pairs += m * n + m * (m + 1) // 2
+        pairs += sum(min(n + i + 1, window) for i in range(m)) if window else m * n + m * (m + 1) // 2
+    q, kv = c["heads"] * c["dim"], c["kv"] * c["dim"]
+    if c["arch"] == "nilatar":
+        lat = c["heads"] * (2 * c["lat"] + NILATAR_ROT)
+        bytes_ += rows * (2 * kv + NILATAR_KV_RANK + NILATAR_ROT) * el
+        flops += 2 * 4.0 * pairs * q + 2.0 * full_pairs * lat + 4.0 * rows * q * c["dim"]
+    else:
+        bytes_ += c["layers"] * (read + rows) * 2 * kv * el
+        flops += c["layers"] * 4.0 * pairs * q
+    bytes_ += rows * (c["width"] * el + 4) + wanted * c["vocab"] * 4
+    return {"bytes": float(bytes_), "flops": float(flops)}
+
+
+def tolerance(case):
+    # about four times the error against 64 bits that was measured
+    if case["dtype"] == "float32":
+        return {"rel": 1e-5}                                             # 2e-6
+    if case["arch"] == "vozinex":
+        # 0.014 for a prompt; of a few decoded rows 0.067 (a router's close call may pick another expert for a row when the
+        # order of a sum changes)
+        return {"rel": 0.25 if case["step"] == "decode" else 0.06}
+    return {"rel": 0.1 if case["layers"] >= 16 else 0.06}                # 0.025 over 32 layers; 0.006 to 0.018 over two to eight
+
+
+# ---------------------------------------------------------------------------------------------- the same in 64 bits
+def _rms(x, w, eps):
+    return x / torch.sqrt((x * x).mean(-1, keepdim=True) + eps) * w
+
+
+def _layer_norm(x, w, b, eps):
+    d = x - x.mean(-1, keepdim=True)
+    return d / torch.sqrt((d * d).mean(-1, keepdim=True) + eps) * w + b
+
+
+def _rotate(x, pos, dims, base):
+    """x [T, heads, d]: i and i + dims / 2 of the first dims dimensions turn by pos base^(-2 i / dims)"""
+    half = dims // 2
+    f = torch.tensor([base ** (-2.0 * i / dims) for i in range(half)], dtype=torch.float64, device=x.device)
+    a = pos[:, None].double() * f
+    c, s = torch.cos(a)[:, None], torch.sin(a)[:, None]
+    u, v = x[..., :half], x[..., half:dims]
+    return torch.cat([u * c - v * s, v * c + u * s, x[..., dims:]], -1)
+
+
+def _rotate_pairs(x, pos, rot):
+    """x [T, heads, dims]: 2 i and 2 i + 1 turn together; the frequencies of a stretched rotation"""
+    dims, base, sc = rot["dims"], rot["base"], rot["scaling"]
+    i = torch.arange(dims // 2, dtype=torch.float64, device=x.device)
+    f = base ** (-2.0 * i / dims)
+
+    def at(turns):
+        return dims * math.log(sc["original"] / (2.0 * math.pi * turns)) / (2.0 * math.log(base))
+    lo, hi = max(math.floor(at(sc["fast"])), 0), min(math.ceil(at(sc["slow"])), dims - 1)
+    ramp = ((i - lo) / max(hi - lo, 0.001)).clamp(0.0, 1.0)
+    f, mult = f / sc["factor"] * ramp + f * (1.0 - ramp), 0.1 * math.log(sc["factor"]) + 1.0
+    a = pos[:, None].double() * f
+    c, s = (torch.cos(a) * mult)[:, None], (torch.sin(a) * mult)[:, None]
+    u, v = x[..., 0::2], x[..., 1::2]
+    return torch.stack([u * c - v * s, v * c + u * s], -1).flatten(-2)
+
+
+def _attend(q, k, v, first, scale, window=None, keep=0, sink=None):
+    """q [T, H, d] at positions first.. over k, v [N, G, .]: softmax over the visible positions"""
+    H, G = q.shape[1], k.shape[1]
+    i = first + torch.arange(q.shape[0], device=q.device)[:, None]
+    j = torch.arange(k.shape[0], device=q.device)[None]
+    hidden = j > i
+    if window is not None:
+        hidden = hidden | ((i - j >= window) & (j >= keep))
+    out = []
+    for h in range(H):
+        s = ((q[:, h] * scale) @ k[:, h // (H // G)].T).masked_fill(hidden, float("-inf"))
+        if sink is not None:
+            s = torch.cat([s, sink[h].expand(s.shape[0], 1)], -1)
+        out.append(torch.softmax(s, -1)[:, :k.shape[0]] @ v[:, h // (H // G)])
+    return torch.stack(out, 1).flatten(1)
+
+
+class _Weights:
+    def __init__(self, case, seed):
+        self.case, self.seed, self.shapes = case, seed, _shapes(case)
+
+    def __call__(self, name):
+        return _tensor(self.case, name, self.shapes[name], self.seed).double()
+
+
+def _past(case, layer, b, n, seed):
+    if n == 0:
+        e = torch.empty(0, case["kv"], case["dim"], dtype=torch.float64, device="cuda")
+        return e, e
+    t = _history(case, layer, b, n, seed).double().permute(1, 0, 3, 2, 4).reshape(2, -1, case["kv"], case["dim"])[:, :n]
+    return t[0], t[1]
+
+
+def _attention(case, seed, layer, ys, cached, weights, rotary, window=None, keep=0, norms=None):
+    """the sequences' rows ys through projections, rotation and attention: the heads side by side"""
+    wq, wk, wv = weights
+    H, G, d, out = case["heads"], case["kv"], case["dim"], []
+    for b, (y, n) in enumerate(zip(ys, cached)):
+        q, k, v = y @ wq.T, y @ wk.T, (y @ wv.T).view(-1, G, d)
+        if norms is not None:
+            q, k = _rms(q, norms[0], case["eps"]), _rms(k, norms[1], case["eps"])
+        pos = n + torch.arange(y.shape[0], device=y.device)
+        q, k = (_rotate(t.view(-1, m, d), pos, rotary, case["theta"]) for t, m in ((q, H), (k, G)))
+        pk, pv = _past(case, layer, b, n, seed)
+        out.append(_attend(q, torch.cat([pk, k]), torch.cat([pv, v]), n, d ** -0.5, window, keep))
+    return torch.cat(out)
+
+
+def _wanted_rows(case, counts):
+    """the wanted places' rows among all sequences' rows"""
+    return [sum(counts[:b]) + place for b, n in enumerate(counts) for place in _want(case, n)]
+
+
+def _exact_llama(case, seed, w, x, counts, cached):
+    eps = case["eps"]
+    for i in range(case["layers"]):
+        p = "model.layers.%d." % i
+        ys = _rms(x, w(p + "input_layernorm.weight"), eps).split(counts)
+        a = p + "self_attn."
+        o = _attention(case, seed, i, ys, cached, [w(a + n + "_proj.weight") for n in "qkv"], case["dim"])
+        x = x + o @ w(a + "o_proj.weight").T
+        y = _rms(x, w(p + "post_attention_layernorm.weight"), eps)
+        h = torch.nn.functional.silu(y @ w(p + "mlp.gate_proj.weight").T) * (y @ w(p + "mlp.up_proj.weight").T)
+        x = x + h @ w(p + "mlp.down_proj.weight").T
+    return _rms(x[_wanted_rows(case, counts)], w("model.norm.weight"), eps) @ w("lm_head.weight").T
+
+
+def _exact_vozinex(case, seed, w, x, counts, cached):
+    eps = case["eps"]
+    for i in range(case["layers"]):
+        p, m = "l%d." % i, "l%d.mix." % i
+        ys = _layer_norm(x, w(p + "norm1"), w(p + "norm1.b"), eps).split(counts)
+        o = _attention(case, seed, i, ys, cached, [w(m + n) for n in "qkv"], case["dim"] // 2, VOZINEX_WINDOW, VOZINEX_KEEP,
+                       (w(m + "q.norm"), w(m + "k.norm")))
+        x = x + o @ w(m + "o").T
+        y = _layer_norm(x, w(p + "norm2"), w(p + "norm2.b"), eps)
+        val, idx = torch.topk(y @ w(p + "mlp.router").T + w(p + "mlp.router.b"), case["top"], -1)
+        share = torch.softmax(val, -1)
+        for e in range(case["experts"]):
+            row, pick = (idx == e).nonzero(as_tuple=True)
+            if len(row):
+                h = torch.relu(y[row] @ w(p + "mlp.e%d.up" % e).T) ** 2 @ w(p + "mlp.e%d.down" % e).T
+                x = x.index_add(0, row, h * share[row, pick][:, None])
+    return _layer_norm(x[_wanted_rows(case, counts)], w("final.norm"), w("final.norm.b"), eps) @ w("head").T
+
+
+def _exact_nilatar(case, seed, w, x, counts, cached):
+    eps, H, G, d = case["eps"], case["heads"], case["kv"], case["dim"]
+    _, latent, lin = _nilatar_mixers(case)
+    kept = []
+    for i in range(case["layers"]):
+        p, m, out = "l%d." % i, "l%d.mix." % i, []
+        for b, y in enumerate(_rms(x, w(p + "norm1"), eps).split(counts)):
+            T = y.shape[0]
+            if i == 1:
+                r, kr, l, pos = NILATAR_ROT, NILATAR_KV_RANK, case["lat"], torch.arange(T, device=y.device)
+                q = (_rms(y @ w(m + "dq").T, w(m + "dq.norm"), eps) @ w(m + "uq").T).view(T, H, l + r)
+                q = torch.cat([q[..., :l], _rotate_pairs(q[..., l:], pos, latent["rot"])], -1)
+                ckv = y @ w(m + "dkv").T
+                c = _rms(ckv[:, :kr], w(m + "dkv.norm"), eps)
+                turned = _rotate_pairs(ckv[:, None, kr:], pos, latent["rot"]).expand(T, H, r)
+                k = torch.cat([(c @ w(m + "uk").T).view(T, H, l), turned], -1)
+                o = _attend(q, k, (c @ w(m + "uv").T).view(T, H, l), 0, latent["scale"])
+            elif i == 2:
+                q, k, v = (torch.nn.functional.silu(y @ w(m + n).T).view(T, H, d) for n in "qkv")
+                decay = torch.tensor(lin["decay"], dtype=torch.float64, device=y.device)
+                S, o = torch.zeros(H, d, d, dtype=torch.float64, device=y.device), []
+                for t in range(T):
+                    S = decay[:, None, None] * S + k[t][:, :, None] * v[t][:, None, :]
+                    o.append((q[t][:, None, :] @ S).flatten())
+                o = _rms(torch.stack(o), w(m + "norm"), eps)
+            else:
+                q = (y @ w(m + "q").T).view(T, H, d)
+                if i == 0:
+                    kept.append([(y @ w(m + n).T).view(T, G, d) for n in "kv"])
+                o = _attend(q, kept[b][0], kept[b][1], 0, d ** -0.5, NILATAR_WINDOW, 0, w(m + "sink"))
+            out.append(o * torch.sigmoid(y @ w(m + "g").T))
+        x = x + torch.cat(out) @ w(m + "o").T * w(p + "ls1")
+        y = _rms(x, w(p + "norm2"), eps)
+        h = torch.nn.functional.gelu(y @ w(p + "mlp.gate").T, approximate="tanh") * (y @ w(p + "mlp.up").T)
+        x = x + h @ w(p + "mlp.down").T * w(p + "ls2")
+    return _rms(x[_wanted_rows(case, counts)], w("final.norm"), eps) @ w("head").T
+
+
+def exact(case, seed):
+    with torch.no_grad():
+        w, tokens = _Weights(case, seed), _tokens(case, seed)
+        embed = "model.embed_tokens.weight" if case["arch"] == "llama" else "embed"
+        ids = torch.tensor([t for s in tokens for t in s], device="cuda")
+        x = _tensor(case, embed, w.shapes[embed], seed)[ids].double()
+        f = {"llama": _exact_llama, "vozinex": _exact_vozinex, "nilatar": _exact_nilatar}[case["arch"]]
+        return f(case, seed, w, x, [len(t) for t in tokens], _cached(case))
