@@ -1,0 +1,180 @@
+// The true 32-bit path's matrix product, C = A W^T, for 32-bit operands whose rows 16-byte copies can take (K, lda and ldw
+// multiples of 4, aligned bases); other operands run k_gemm_simt (generic.cu). The sums are the same: every output adds its
+// K terms one after the other with 32-bit fused multiply-adds, so its bits do not depend on the kernel, the tile it lands in
+// or the number of rows.
+//
+// What bounds it is the FMA rate for prompts (74 TFLOP/s at 1.96 GHz) and the weights' way from memory for a few rows.
+// k_gemm_simt's 4 x 4 outputs a thread cost eight scalar shared-memory reads for 16 FMAs. Here a thread holds TM x TN
+// outputs and reads four K elements of a row per access (TM + TN 16-byte reads for 4 TM TN FMAs); rows lie BK + 4 floats
+// apart in shared memory, so that the eight rows a quarter-warp reads fall into different banks; tiles arrive by
+// asynchronous copies STAGES - 1 blocks ahead, the first weights before the wait on the kernel that writes A.
+#include "common.cuh"
+
+__device__ __forceinline__ void kb_cp16(uint32_t dst, const void* src, bool on) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(on ? 16 : 0) : "memory");
+}
+template <int BM, int BN, int TM, int TN, int BK, int STAGES>
+struct F32Tile {
+    static constexpr int THREADS = (BM / TM) * (BN / TN);
+    static constexpr int LD = BK + 4;
+    static constexpr int STAGE = (BM + BN) * LD;                       // floats
+    static constexpr int SMEM = STAGES * STAGE * 4;
+};
+template <int BM, int BN, int TM, int TN, int BK, int STAGES>
+__global__ void __launch_bounds__((BM / TM) * (BN / TN)) k_gemm_f32(const float* KB_STEP_DATA A, const float* __restrict__ W,
+        float* __restrict__ C, int M, int N, int K, int lda, int ldw, int ldc) {
+    using S = F32Tile<BM, BN, TM, TN, BK, STAGES>;
+    constexpr int NT = S::THREADS, LD = S::LD, PIECES = BK / 4;
+    // a warp covers WM x WN threads of the tile: eight neighbouring rows of W (one conflict-free read), the others share A
+    constexpr int NX = BN / TN, WN = NX < 8 ? NX : 8, WM = 32 / WN;
+    static_assert(BK % 4 == 0 && NX % WN == 0 && (BM / TM) % WM == 0, "a warp's threads tile the block");
+    extern __shared__ __align__(16) float smf[];
+    kb_pdl_launch();
+    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tx = (warp % (NX / WN)) * WN + lane % WN, ty = (warp / (NX / WN)) * WM + lane / WN;
+    const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(smf);
+    const int n_blocks = (K + BK - 1) / BK;
+    auto fetch_w = [&](int b) {
+        const uint32_t at = sbase + ((b % STAGES) * S::STAGE + BM * LD) * 4;
+#pragma unroll
+        for (int e = tid; e < BN * PIECES; e += NT) {
+            const int r = e / PIECES, c = e % PIECES, k = b * BK + c * 4;
+            const bool on = n0 + r < N && k < K;
+            kb_cp16(at + (r * LD + c * 4) * 4, on ? W + (size_t)(n0 + r) * ldw + k : W, on);
+        }
+    };
+    auto fetch_a = [&](int b) {
+        const uint32_t at = sbase + (b % STAGES) * S::STAGE * 4;
+#pragma unroll
+        for (int e = tid; e < BM * PIECES; e += NT) {
+            const int r = e / PIECES, c = e % PIECES, k = b * BK + c * 4;
+            const bool on = m0 + r < M && k < K;
+            kb_cp16(at + (r * LD + c * 4) * 4, on ? A + (size_t)(m0 + r) * lda + k : A, on);
+        }
+    };
+    // the weights of the first blocks are requested before the wait on the kernel that writes A
+#pragma unroll
+    for (int b = 0; b < STAGES - 1; b++)
+        if (b < n_blocks) fetch_w(b);
+    kb_pdl_wait();
+#pragma unroll
+    for (int b = 0; b < STAGES - 1; b++) {
+        if (b < n_blocks) fetch_a(b);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    float acc[TM][TN];
+#pragma unroll
+    for (int i = 0; i < TM; i++)
+#pragma unroll
+        for (int j = 0; j < TN; j++) acc[i][j] = 0.0f;
+    for (int b = 0; b < n_blocks; b++) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
+        __syncthreads();                             // block b is there for everybody, block b - 1's stage is free
+        if (b + STAGES - 1 < n_blocks) {
+            fetch_w(b + STAGES - 1);
+            fetch_a(b + STAGES - 1);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        const float* sa = smf + (b % STAGES) * S::STAGE + ty * LD;
+        const float* sw = smf + (b % STAGES) * S::STAGE + (BM + tx) * LD;
+        // (elements past K are zero in both tiles: they leave a sum as it is)
+#pragma unroll
+        for (int k = 0; k < BK; k += 4) {
+            float4 a[TM], w[TN];
+#pragma unroll
+            for (int i = 0; i < TM; i++) a[i] = *(const float4*)(sa + i * (BM / TM) * LD + k);
+#pragma unroll
+            for (int j = 0; j < TN; j++) w[j] = *(const float4*)(sw + j * NX * LD + k);
+#pragma unroll
+            for (int i = 0; i < TM; i++)
+#pragma unroll
+                for (int j = 0; j < TN; j++) acc[i][j] = fmaf(a[i].x, w[j].x, acc[i][j]);
+#pragma unroll
+            for (int i = 0; i < TM; i++)
+#pragma unroll
+                for (int j = 0; j < TN; j++) acc[i][j] = fmaf(a[i].y, w[j].y, acc[i][j]);
+#pragma unroll
+            for (int i = 0; i < TM; i++)
+#pragma unroll
+                for (int j = 0; j < TN; j++) acc[i][j] = fmaf(a[i].z, w[j].z, acc[i][j]);
+#pragma unroll
+            for (int i = 0; i < TM; i++)
+#pragma unroll
+                for (int j = 0; j < TN; j++) acc[i][j] = fmaf(a[i].w, w[j].w, acc[i][j]);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < TM; i++) {
+        const int m = m0 + ty + i * (BM / TM);
+        if (m >= M) continue;
+#pragma unroll
+        for (int j = 0; j < TN; j++) {
+            const int n = n0 + tx + j * NX;
+            if (n < N) C[(size_t)m * ldc + n] = acc[i][j];
+        }
+    }
+}
+
+template <int BM, int BN, int TM, int TN, int BK, int STAGES>
+static int launch_f32(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw, int ldc,
+                      cudaStream_t st) {
+    using S = F32Tile<BM, BN, TM, TN, BK, STAGES>;
+    auto kern = k_gemm_f32<BM, BN, TM, TN, BK, STAGES>;
+    static char once_tag;
+    if (S::SMEM > 48 * 1024 && kb_first_use(&once_tag)) {
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::SMEM);
+        if (e != cudaSuccess) return (int)e;
+    }
+    kb_launch(kern, dim3((N + BN - 1) / BN, (M + BM - 1) / BM), S::THREADS, S::SMEM, st, A, W, C, M, N, K, lda, ldw, ldc);
+    KB_LAUNCH_RET();
+}
+
+// The tiles, and what a unit of 1024 K elements takes on an SM, in microseconds: alone, and beside enough others (measured
+// at N = 32768; large products reach 44 TFLOP/s). Few units want small tiles: 514 x 1024 outputs over K = 1024 take 80 us in
+// tiles of 64 x 128 and 61 to 69 us in tiles of 32 x 32 or 16 x 64; four rows of 5632 columns 70 against 14 us.
+struct F32Choice { int bm, bn; float alone, each; };
+static const F32Choice kF32Tiles[] = {{64, 128, 70.f, 54.f}, {64, 64, 37.f, 28.f}, {32, 64, 24.f, 15.3f}, {32, 32, 17.f, 9.4f},
+                                      {16, 64, 18.f, 10.6f}, {16, 32, 13.4f, 9.7f}, {8, 64, 14.f, 10.5f}, {4, 64, 11.8f, 8.5f}};
+
+// the tile of the least estimated time: whole rounds of units while they are few; and units beyond the first on an SM share
+// it unevenly (six tenths of a lone unit's time, measured)
+static int f32_tile(int M, int N) {
+    static int sms = 0;
+    if (!sms) {
+        int dev = 0;
+        cudaGetDevice(&dev);
+        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
+    }
+    int best = 0;
+    float best_cost = 0.0f;
+    for (int i = 0; i < (int)(sizeof(kF32Tiles) / sizeof(kF32Tiles[0])); i++) {
+        const F32Choice& t = kF32Tiles[i];
+        const long long units = (long long)((M + t.bm - 1) / t.bm) * ((N + t.bn - 1) / t.bn);
+        const float rounds = units <= 4 * sms ? (float)((units + sms - 1) / sms) : (float)units / (float)sms;
+        const float cost = (rounds * t.each > t.alone ? rounds * t.each : t.alone) + (units > 90 ? 0.6f * t.alone : 0.0f);
+        if (i == 0 || cost < best_cost) {
+            best = i;
+            best_cost = cost;
+        }
+    }
+    return best;
+}
+
+// tile: an index of kF32Tiles, or -1 to choose
+extern "C" int kb_gemm_f32(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw, int ldc, int tile,
+                           cudaStream_t st) {
+    if (M <= 0 || N <= 0) return 0;
+    if (K % 4 || lda % 4 || ldw % 4 || ((uintptr_t)A & 15) || ((uintptr_t)W & 15)) return (int)cudaErrorInvalidValue;
+    switch (tile < 0 ? f32_tile(M, N) : tile) {
+        case 0: return launch_f32<64, 128, 8, 8, 16, 4>(A, W, C, M, N, K, lda, ldw, ldc, st);
+        case 1: return launch_f32<64, 64, 8, 4, 32, 2>(A, W, C, M, N, K, lda, ldw, ldc, st);
+        case 2: return launch_f32<32, 64, 4, 4, 32, 2>(A, W, C, M, N, K, lda, ldw, ldc, st);
+        case 3: return launch_f32<32, 32, 4, 2, 32, 3>(A, W, C, M, N, K, lda, ldw, ldc, st);
+        case 4: return launch_f32<16, 64, 4, 2, 32, 3>(A, W, C, M, N, K, lda, ldw, ldc, st);
+        case 5: return launch_f32<16, 32, 2, 1, 64, 3>(A, W, C, M, N, K, lda, ldw, ldc, st);
+        case 6: return launch_f32<8, 64, 2, 1, 64, 3>(A, W, C, M, N, K, lda, ldw, ldc, st);
+        case 7: return launch_f32<4, 64, 1, 1, 64, 4>(A, W, C, M, N, K, lda, ldw, ldc, st);
+        default: return (int)cudaErrorInvalidValue;
+    }
+}

@@ -661,9 +661,15 @@ __global__ void __launch_bounds__(256) k_gemm_simt(const TA* KB_STEP_DATA A, con
     }
 }
 
+extern "C" int kb_gemm_f32(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw, int ldc, int tile,
+                           cudaStream_t st);
+
 extern "C" int kb_gemm_simt(const void* A, int adtype, const void* W, int wdtype, void* C, int cdtype, int M, int N,
                             int K, int lda, int ldw, int ldc, cudaStream_t st) {
     if (M <= 0 || N <= 0) return 0;
+    if (adtype == KB_F32 && wdtype == KB_F32 && cdtype == KB_F32 && K > 0 && K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 &&
+        ((uintptr_t)A & 15) == 0 && ((uintptr_t)W & 15) == 0)
+        return kb_gemm_f32((const float*)A, (const float*)W, (float*)C, M, N, K, lda, ldw, ldc, -1, st);    // the same bits
     dim3 grid((N + GS_BN - 1) / GS_BN, (M + GS_BM - 1) / GS_BM);
 #define KB_G(TA, TW, TC) \
     kb_launch(k_gemm_simt<TA, TW, TC>, grid, 256, 0, st, (const TA*)A, (const TW*)W, (TC*)C, M, N, K, lda, ldw, ldc)
@@ -1185,6 +1191,11 @@ __global__ void __launch_bounds__(128) k_attn_generic(const T* KB_STEP_DATA q, i
     }
 }
 
+bool kb_attn_rows_takes(const void* q, int ldq, const void* out, int ldo, const void* pool, int hd, int vd);
+int kb_attn_rows(const float* q, int ldq, float* out, int ldo, const int* pos, const int* seq, const int* slot, int T, int nkv,
+                 int group, int hd, float scale, int window, int keep_first, const KbCacheView& cv, int* status,
+                 const float* sink, const float* gate, int ldg, int chunk, float cap, int vd, cudaStream_t st);
+
 extern "C" int kb_attn_generic(const void* q, int dtype, int ldq, void* out, int ldo, const int* pos, const int* seq,
                                const int* slot, int T, int nh, int nkv, int hd, float scale, int window, void* pool,
                                const int* table, int table_stride, int n_pages, int* status, cudaStream_t st,
@@ -1198,6 +1209,10 @@ extern "C" int kb_attn_generic(const void* q, int dtype, int ldq, void* out, int
     if (vd <= 0) vd = hd;
     if (vd > hd) return (int)cudaErrorInvalidValue;
     KbCacheView cv{pool, table, table_stride, n_pages, nkv, hd, one_plane};
+    // 32-bit heads of up to 128 elements: the same arithmetic over tiles that rows share (attn_rows.cu)
+    if (dtype == KB_F32 && kb_attn_rows_takes(q, ldq, out, ldo, pool, hd, vd))
+        return kb_attn_rows((const float*)q, ldq, (float*)out, ldo, pos, seq, slot, T, nkv, nh / nkv, hd, scale, window,
+                            keep_first, cv, status, sink, (const float*)gate, ldg, chunk, cap, vd, st);
     long long items = (long long)T * nh;
     int grid = (int)((items + 3) / 4);
     if (dtype == KB_F32)

@@ -54,6 +54,7 @@ _SIGS = {
                        c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p],
     "kb_gemm_simt": [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
                      c_void_p],
+    "kb_gemm_f32": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p],
     "kb_rope_store": [c_void_p, c_int, c_int, c_longlong, c_int, c_void_p, c_int, c_int, c_void_p, c_int, c_void_p,
                       c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_int, c_void_p,
                       c_void_p, c_void_p],
@@ -759,6 +760,17 @@ def gemm_simt(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
     assert a.stride(1) == 1 and w.stride(1) == 1 and out.stride(1) == 1
     _check(load().kb_gemm_simt(_p(a), dt(a), _p(w), dt(w), _p(out), dt(out), M, N, K, a.stride(0), w.stride(0),
                                out.stride(0), _stream()), "gemm_simt")
+
+
+def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, tile: int = -1) -> None:
+    """``gemm_simt`` of float32 operands whose rows are aligned for 16-byte copies, on a given tile of the kernel it takes
+    for them (-1: the one it would choose); every tile gives the same bits"""
+    _need_cuda(a, w, out)
+    (M, K), N = a.shape, w.shape[0]
+    assert a.dtype == w.dtype == out.dtype == torch.float32 and w.shape[1] == K and out.shape == (M, N)
+    assert a.stride(1) == 1 and w.stride(1) == 1 and out.stride(1) == 1
+    _check(load().kb_gemm_f32(_p(a), _p(w), _p(out), M, N, K, a.stride(0), w.stride(0), out.stride(0), tile, _stream()),
+           "gemm_f32")
 
 
 @functools.lru_cache(maxsize=1)

@@ -1,0 +1,96 @@
+"""The 32-bit path's tiled product and tiled attention against the general kernels they stand in for: the same sums in
+the same order, so the same bits, at edges of tiles and with every option of the attention."""
+import random
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def K():
+    from kindi_b200.kernels import lib
+    lib.load()
+    return lib
+
+
+@pytest.mark.parametrize("tile", [-1] + list(range(8)))
+@pytest.mark.parametrize("M,N,K_", [(1, 64, 4), (5, 127, 68), (16, 33, 1024), (65, 129, 140), (130, 260, 60), (257, 96, 2816)])
+def test_every_tile_gives_the_general_kernels_bits(K, M, N, K_, tile):
+    g = torch.Generator(device="cuda").manual_seed(M * 1000 + N + K_)
+    a = torch.randn(M, K_, device="cuda", generator=g)
+    w = torch.randn(N, K_, device="cuda", generator=g)
+    odd = torch.empty(M, K_ + 1, device="cuda")[:, :K_]            # rows that no 16-byte copy takes: the general kernel
+    odd.copy_(a)
+    want, got = torch.empty(M, N, device="cuda"), torch.full((M, N + 3), float("nan"), device="cuda")
+    K.gemm_simt(odd, w, want)
+    K.gemm_f32(a, w, got[:, :N], tile)
+    assert torch.equal(got[:, :N], want) and bool(got[:, N:].isnan().all())
+    wide = torch.randn(M, K_ + 8, device="cuda", generator=g)      # a row stride of its own
+    wide[:, 4:4 + K_] = a
+    K.gemm_f32(wide[:, 4:4 + K_], w, got[:, :N], tile)
+    assert torch.equal(got[:, :N], want)
+
+
+OPTIONS = [dict(), dict(window=37), dict(window=70, keep_first=5), dict(window=64, keep_first=130), dict(chunk=48),
+           dict(softcap=3.0), dict(sink=True, gate=True), dict(v_dim=24), dict(one_plane=True, v_dim=20)]
+
+
+@pytest.mark.parametrize("options", OPTIONS)
+@pytest.mark.parametrize("nh,nkv,hd", [(4, 2, 32), (5, 1, 128), (3, 3, 44), (40, 2, 64)])
+def test_attention_over_shared_tiles_gives_the_general_kernels_bits(K, nh, nkv, hd, options):
+    opt = dict(options)
+    use_sink, use_gate, one = opt.pop("sink", False), opt.pop("gate", False), opt.pop("one_plane", False)
+    if one and nkv != 1:
+        nh, nkv = 6, 1
+    rng = random.Random(nh * 100 + hd)
+    q_lens, kv_lens = [1, 33, 7, 1], [1, 200, 140, 97]
+    vd = opt.get("v_dim") or hd
+    n_pages = 16
+    g = torch.Generator(device="cuda").manual_seed(hd)
+    pool = torch.randn(n_pages, 1 if one else 2, nkv, 64, hd, device="cuda", generator=g)
+    order = list(range(n_pages))
+    rng.shuffle(order)
+    table = torch.full((4, 8), -1, dtype=torch.int32)
+    pos, seq = [], []
+    for b, (ql, kl) in enumerate(zip(q_lens, kv_lens)):
+        for i in range(-(-kl // 64)):
+            table[b, i] = order.pop()
+        pos += list(range(kl - ql, kl))
+        seq += [b] * ql
+    pos += [-1, -1]                                                 # padding rows of a recorded step
+    seq += [0, 0]
+    T = len(pos)
+    dev = lambda x: torch.tensor(x, dtype=torch.int32).cuda()      # noqa: E731
+    q = torch.randn(T, nh * hd, device="cuda", generator=g)
+    sink = torch.randn(nh, device="cuda", generator=g) if use_sink else None
+    gate = torch.randn(T, nh * vd, device="cuda", generator=g) if use_gate else None
+
+    def go(out, cache):
+        st = torch.zeros(1, dtype=torch.int32, device="cuda")
+        K.attn_generic(q, out, dev(pos), dev(seq), dev([0, 1, 2, 3]), nh, nkv, hd, 0.2, opt.get("window", 0), cache,
+                       table.cuda(), n_pages, st, opt.get("keep_first", 0), sink, gate, opt.get("chunk", 0),
+                       opt.get("softcap", 0.0), vd)
+        assert int(st.item()) == 0
+        return out
+    # (rows of an odd stride run the general kernel)
+    want = go(torch.full((T, nh * vd + 1), 7.0, device="cuda")[:, :nh * vd], pool)
+    got = go(torch.full((T, nh * vd), 7.0, device="cuda"), pool)
+    assert torch.equal(got, want) and bool((got[-2:] == 7.0).all())
+    # a NaN at a position that only later rows see stays out of the earlier ones
+    pool2 = pool.clone()
+    pool2[int(table[1, 190 // 64]), :, :, 190 % 64] = float("nan")
+    want2 = go(torch.empty(T, nh * vd + 1, device="cuda")[:, :nh * vd], pool2)[:T - 2]
+    got2 = go(torch.empty(T, nh * vd, device="cuda"), pool2)[:T - 2]
+    assert torch.equal(got2.isnan(), want2.isnan()) and torch.equal(got2.nan_to_num(1.0), want2.nan_to_num(1.0))
+
+
+def test_an_unmapped_page_is_reported_only_where_a_row_sees_it(K):
+    pool = torch.randn(4, 2, 1, 64, 32, device="cuda")
+    q, out = torch.randn(2, 32, device="cuda"), torch.empty(2, 32, device="cuda")
+    dev = lambda x: torch.tensor(x, dtype=torch.int32).cuda()      # noqa: E731
+    for row, window, bad in (([-1, 1, 2], 60, False), ([-1, 1, 2], 0, True), ([9, 1, 2], 0, True), ([0, 1, -1], 0, True)):
+        st = torch.zeros(1, dtype=torch.int32, device="cuda")
+        K.attn_generic(q, out, dev([130, 131]), dev([0, 0]), dev([0]), 1, 1, 32, 0.2, window, pool, dev([row]), 4, st)
+        assert (int(st.item()) == K.ST_BAD_PAGE) == bad
