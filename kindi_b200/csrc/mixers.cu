@@ -762,135 +762,6 @@ __global__ void __launch_bounds__(256) k_decay_chunk(const TIN* KB_STEP_DATA in,
     }
 }
 
-// chunked form: C = tokens of a chunk, nc_max = the most chunks a sequence of this step can have (the longest
-// sequence's; an upper bound is fine), P (float [B][H][nc_max][dv][d]) and S0 (float [B][H][dv][d]) scratch
-// The two passes with a THREAD per column of the state (key sizes up to 128): the thread holds its column's D
-// elements in registers, so a token's output is a private sum (no exchange between lanes), k and q of a token are
-// read from shared memory as broadcasts of four, and a block's threads write 128 neighbouring outputs. About a third
-// of the instructions per token of the warp-per-column form above, which stays for larger key sizes.
-#define DK_TILE 16
-#define DK_COLS 128
-template <typename TIN, bool OUT, int D>
-__global__ void __launch_bounds__(DK_COLS) k_decay_chunk_col(const TIN* KB_STEP_DATA in, int n_planes,
-        size_t plane_stride, int ld_in, int H, int d, int dv, const float* __restrict__ decay,
-        const int* __restrict__ q_start, const int* __restrict__ slot, float* state, float* P, float* S0,
-        float* __restrict__ out, int ldo, int C, int nc_max) {
-    extern __shared__ __align__(16) float smc[];
-    float* qs = smc;                                  // [DK_TILE][D] (zeros past d)
-    float* ks = qs + DK_TILE * D;                     // [DK_TILE][D]
-    float* vs = ks + DK_TILE * D;                     // [DK_TILE][DK_COLS]
-    kb_pdl_launch();
-    const int b = blockIdx.x / H, h = blockIdx.x % H, c = blockIdx.z;
-    const int e0 = blockIdx.y * DK_COLS, e = e0 + threadIdx.x;
-    const bool live = e < dv;
-    const int r0 = q_start[b], r1 = q_start[b + 1];
-    const int nc = (r1 - r0 + C - 1) / C;
-    if (c >= nc) return;
-    const bool last = c == nc - 1;
-    const float lam = decay[h];
-    const size_t bh = (size_t)b * H + h;
-    float* srow = state + (((size_t)slot[b] * H + h) * dv + (live ? e : 0)) * d;
-    float* s0row = S0 + (bh * dv + (live ? e : 0)) * d;
-    float* prow = P + ((bh * nc_max + c) * dv + (live ? e : 0)) * d;
-    kb_pdl_wait();
-    float S[D];
-    if (!OUT) {
-        if (c == 0 && live)
-            for (int j = 0; j < d; j++) s0row[j] = srow[j];
-        if (last) return;
-#pragma unroll
-        for (int j = 0; j < D; j++) S[j] = 0.0f;
-    } else {
-#pragma unroll
-        for (int j = 0; j < D; j++) S[j] = (live && j < d) ? prow[j] : 0.0f;
-    }
-    const int ra = r0 + c * C, rz = min(ra + C, r1);
-    const size_t oq = (size_t)h * d, ok = (size_t)H * d + (size_t)h * d, ov = (size_t)2 * H * d + (size_t)h * dv;
-    // (silu(0) = 0: a zero piece past the row's end or past d stages zeros)
-    const bool vec8 = sizeof(TIN) == 2 && n_planes == 1 && d % 8 == 0 && ld_in % 8 == 0 && ((uintptr_t)in & 15) == 0;
-    for (int t0 = ra; t0 < rz; t0 += DK_TILE) {
-        const int n = min(DK_TILE, rz - t0);
-        if (vec8) {
-            // bf16 rows whose heads start on 16-byte boundaries: eight elements a load, all of a thread's loads in
-            // flight before the first is used
-            constexpr int PER = (DK_TILE * D / 8 + DK_COLS - 1) / DK_COLS;
-            uint4 rq[PER], rk[PER];
-#pragma unroll
-            for (int u = 0; u < PER; u++) {
-                const int idx = (threadIdx.x + DK_COLS * u) * 8, t = idx / D, j = idx % D;
-                rq[u] = rk[u] = make_uint4(0u, 0u, 0u, 0u);
-                if (idx < DK_TILE * D && t < n && j < d) {
-                    const bf16* src = (const bf16*)in + (size_t)(t0 + t) * ld_in;
-                    if (OUT) rq[u] = *(const uint4*)(src + oq + j);
-                    rk[u] = *(const uint4*)(src + ok + j);
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < PER; u++) {
-                const int idx = (threadIdx.x + DK_COLS * u) * 8;
-                if (idx >= DK_TILE * D) continue;
-                const __nv_bfloat162* q2 = (const __nv_bfloat162*)&rq[u];
-                const __nv_bfloat162* k2 = (const __nv_bfloat162*)&rk[u];
-#pragma unroll
-                for (int w = 0; w < 4; w++) {
-                    const float2 kf = __bfloat1622float2(k2[w]);
-                    ks[idx + 2 * w] = mx_silu_fast(kf.x);
-                    ks[idx + 2 * w + 1] = mx_silu_fast(kf.y);
-                    if (OUT) {
-                        const float2 qf = __bfloat1622float2(q2[w]);
-                        qs[idx + 2 * w] = mx_silu_fast(qf.x);
-                        qs[idx + 2 * w + 1] = mx_silu_fast(qf.y);
-                    }
-                }
-            }
-        } else {
-            for (int idx = threadIdx.x; idx < DK_TILE * D; idx += DK_COLS) {
-                const int t = idx / D, j = idx % D;
-                float qv = 0.0f, kv = 0.0f;
-                if (t < n && j < d) {
-                    const TIN* src = in + (size_t)(t0 + t) * ld_in;
-                    if (OUT) qv = mx_silu_fast(mx_rd<TIN>(src, n_planes, plane_stride, oq + j));
-                    kv = mx_silu_fast(mx_rd<TIN>(src, n_planes, plane_stride, ok + j));
-                }
-                if (OUT) qs[idx] = qv;
-                ks[idx] = kv;
-            }
-        }
-        for (int t = 0; t < n; t++)
-            vs[t * DK_COLS + threadIdx.x] =
-                live ? mx_silu_fast(mx_rd<TIN>(in + (size_t)(t0 + t) * ld_in, n_planes, plane_stride, ov + e)) : 0.0f;
-        __syncthreads();
-        for (int t = 0; t < n; t++) {
-            const float v = vs[t * DK_COLS + threadIdx.x];
-            float p0 = 0.0f, p1 = 0.0f;
-#pragma unroll
-            for (int j = 0; j < D; j += 4) {
-                const float4 k4 = *(const float4*)(ks + t * D + j);
-                S[j] = fmaf(lam, S[j], __fmul_rn(k4.x, v));
-                S[j + 1] = fmaf(lam, S[j + 1], __fmul_rn(k4.y, v));
-                S[j + 2] = fmaf(lam, S[j + 2], __fmul_rn(k4.z, v));
-                S[j + 3] = fmaf(lam, S[j + 3], __fmul_rn(k4.w, v));
-                if (OUT) {
-                    const float4 q4 = *(const float4*)(qs + t * D + j);
-                    p0 = fmaf(S[j], q4.x, p0);
-                    p1 = fmaf(S[j + 1], q4.y, p1);
-                    p0 = fmaf(S[j + 2], q4.z, p0);
-                    p1 = fmaf(S[j + 3], q4.w, p1);
-                }
-            }
-            if (OUT && live) out[(size_t)(t0 + t) * ldo + (size_t)h * dv + e] = p0 + p1;
-        }
-        __syncthreads();
-    }
-    if (live && (!OUT || last)) {
-        float* dst = OUT ? srow : prow;
-#pragma unroll
-        for (int j = 0; j < D; j++)
-            if (j < d) dst[j] = S[j];
-    }
-    (void)s0row;
-}
-
 // between the two passes: P[c] (a chunk's own contribution) becomes the state BEFORE chunk c, element by element:
 // S = the state the sequence came with; for c = 0, 1, ...: (P[c], S) <- (S, decay^C S + P[c])
 __global__ void __launch_bounds__(256) k_decay_prefix(int H, int d, int dv, const float* __restrict__ decay,
@@ -919,52 +790,40 @@ __global__ void __launch_bounds__(256) k_decay_prefix(int H, int d, int dv, cons
     }
 }
 
+// (decay_chunk.cu)
+int kb_decay_tiles(const void* in, int in_dtype, int n_planes, size_t plane_stride, int ld_in, int B, int H, int d, int dv,
+                   const float* decay, const int* q_start, const int* slot, float* state, float* P, float* out, int ldo, int C,
+                   int nc_max, cudaStream_t st);
+
+// chunked form: C = tokens of a chunk, nc_max = the most chunks a sequence of this step can have (the longest
+// sequence's; an upper bound is fine), P (float [B][H][nc_max][dv][d]) and S0 (float [B][H][dv][d]) scratch. Key sizes up to
+// 128 run as matrix products over tiles of tokens (decay_chunk.cu), larger ones with a warp per column of the state
 extern "C" int kb_decay_chunked(const void* in, int in_dtype, int n_planes, long long plane_stride, int ld_in, int B,
                                 int H, int d, int dv, const float* decay, const int* q_start, const int* slot,
                                 float* state, float* P, float* S0, float* out, int ldo, int C, int nc_max,
                                 cudaStream_t st) {
     if (B <= 0 || H <= 0 || nc_max <= 0) return 0;
     if (d > 32 * DS_MAX_DPL || d <= 0 || dv <= 0 || C <= 0 || nc_max > 65535) return (int)cudaErrorInvalidValue;
+    if (d <= 128)
+        return kb_decay_tiles(in, in_dtype, n_planes, (size_t)plane_stride, ld_in, B, H, d, dv, decay, q_start, slot, state, P, out,
+                              ldo, C, nc_max, st);
     dim3 grid(B * H, (dv + DC_COLS - 1) / DC_COLS, nc_max);
-    dim3 gk(B * H, (dv + DK_COLS - 1) / DK_COLS, nc_max);
     dim3 gs(B * H, (unsigned)((dv * d + 255) / 256 < 64 ? (dv * d + 255) / 256 : 64));
-#define KB_DC2(TIN, DPL)                                                                                            \
+#define KB_DC(TIN)                                                                                                  \
     do {                                                                                                            \
-        const size_t sm = (size_t)(2 * DC_TILE * 32 * DPL + DC_TILE * DC_COLS) * sizeof(float);                     \
-        kb_launch(k_decay_chunk<TIN, false, DPL>, grid, 256, sm, st, (const TIN*)in, n_planes,                     \
+        const size_t sm = (size_t)(2 * DC_TILE * 256 + DC_TILE * DC_COLS) * sizeof(float);                          \
+        kb_launch(k_decay_chunk<TIN, false, 8>, grid, 256, sm, st, (const TIN*)in, n_planes,                       \
                   (size_t)plane_stride, ld_in, H, d, dv, decay, q_start, slot, state, P, S0, out, ldo, C, nc_max);  \
         cudaError_t e = cudaGetLastError();                                                                         \
         if (e != cudaSuccess) return (int)e;                                                                        \
         kb_launch(k_decay_prefix, gs, 256, 0, st, H, d, dv, decay, q_start, P, (const float*)S0, C, nc_max);        \
         e = cudaGetLastError();                                                                                     \
         if (e != cudaSuccess) return (int)e;                                                                        \
-        kb_launch(k_decay_chunk<TIN, true, DPL>, grid, 256, sm, st, (const TIN*)in, n_planes,                      \
+        kb_launch(k_decay_chunk<TIN, true, 8>, grid, 256, sm, st, (const TIN*)in, n_planes,                        \
                   (size_t)plane_stride, ld_in, H, d, dv, decay, q_start, slot, state, P, S0, out, ldo, C, nc_max);  \
-    } while (0)
-#define KB_DK2(TIN, D)                                                                                              \
-    do {                                                                                                            \
-        const size_t sm = (size_t)(2 * DK_TILE * D + DK_TILE * DK_COLS) * sizeof(float);                            \
-        kb_launch(k_decay_chunk_col<TIN, false, D>, gk, DK_COLS, sm, st, (const TIN*)in, n_planes,                  \
-                  (size_t)plane_stride, ld_in, H, d, dv, decay, q_start, slot, state, P, S0, out, ldo, C, nc_max);  \
-        cudaError_t e = cudaGetLastError();                                                                         \
-        if (e != cudaSuccess) return (int)e;                                                                        \
-        kb_launch(k_decay_prefix, gs, 256, 0, st, H, d, dv, decay, q_start, P, (const float*)S0, C, nc_max);        \
-        e = cudaGetLastError();                                                                                     \
-        if (e != cudaSuccess) return (int)e;                                                                        \
-        kb_launch(k_decay_chunk_col<TIN, true, D>, gk, DK_COLS, sm, st, (const TIN*)in, n_planes,                   \
-                  (size_t)plane_stride, ld_in, H, d, dv, decay, q_start, slot, state, P, S0, out, ldo, C, nc_max);  \
-    } while (0)
-#define KB_DC(TIN)                          \
-    do {                                    \
-        if (d <= 32) KB_DK2(TIN, 32);       \
-        else if (d <= 64) KB_DK2(TIN, 64);  \
-        else if (d <= 128) KB_DK2(TIN, 128);\
-        else KB_DC2(TIN, 8);                \
     } while (0)
     if (in_dtype == KB_F32) KB_DC(float);
     else KB_DC(bf16);
-#undef KB_DK2
-#undef KB_DC2
 #undef KB_DC
     KB_LAUNCH_RET();
 }
