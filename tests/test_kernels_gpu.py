@@ -617,3 +617,34 @@ def test_rotation_angles_of_a_step_are_the_kernels_own(K):
     first_pad = 1000 + T - 3                                           # the first position that no row stores
     assert float(res[1][1][first_pad // 64, :, :, first_pad % 64:].abs().sum()) == 0.0
     assert float(res[1][1][first_pad // 64, :, :, first_pad % 64 - 1].abs().sum()) > 0.0
+
+
+@pytest.mark.parametrize("kind", ["rms", "layer"])
+@pytest.mark.parametrize("T,E,planes,scaled", [(160, 1024, 1, False), (161, 1028, 2, True), (163, 2048, 5, False),
+                                               (201, 2052, 0, False), (177, 3072, 1, True), (160, 3076, 3, False),
+                                               (171, 4096, 2, False), (163, 4100, 1, False), (160, 6144, 9, True), (160, 6148, 1, False)])
+def test_norm_of_rows_shared_by_warps(K, kind, T, E, planes, scaled):
+    """every split of a row over warps, at its widest and just above, with rows that do not fill the last block, gains that are
+    aligned and gains that are not (those keep the block per row)"""
+    if kind == "layer" and scaled:
+        scaled = False
+    g = torch.Generator(device="cuda").manual_seed(T * 10000 + E)
+    x0 = torch.randn(T, E, device="cuda", generator=g)
+    d = torch.randn(planes, T, E, device="cuda", generator=g) * 0.3 if planes else None
+    both = torch.randn(2, E + 2, device="cuda", generator=g)
+    for wdtype, at in ((torch.float32, 0), (torch.bfloat16, 0), (torch.bfloat16, 1)):
+        w, b = (both[0] * 0.1 + 1).to(wdtype)[at:at + E], both[1].to(wdtype)[at:at + E]
+        ls = (both[1] + 1).to(wdtype)[:E].contiguous() if scaled and planes else None
+        x, y, st = x0.clone(), torch.empty(T, E, device="cuda", dtype=torch.bfloat16), _status()
+        branch = d.double().sum(0) if planes else torch.zeros(T, E, device="cuda", dtype=torch.float64)
+        v = x0.double() + (branch * ls.double() if ls is not None else branch)
+        if kind == "rms":
+            K.add_rmsnorm(x, d, w, 1e-5, y, None, d is not None, st, ls)
+            want = v / torch.sqrt((v * v).mean(-1, keepdim=True) + 1e-5) * w.double()
+        else:
+            K.add_layernorm(x, d, w, b, 1e-5, y, None, d is not None, st)
+            u = v - v.mean(-1, keepdim=True)
+            want = u / torch.sqrt((u * u).mean(-1, keepdim=True) + 1e-5) * w.double() + b.double()
+        assert _rel(x, v) < 1e-6
+        # one bf16 rounding of the result, 2^-9 of a value
+        assert float(((y.double() - want).abs() / (want.abs() + 1e-2)).max()) < 2 ** -8
