@@ -52,6 +52,18 @@ class FreeList:
         self._held[i] = True
         return i
 
+    def take_many(self, n: int) -> List[int]:
+        """what n calls of ``take`` hand out, or CacheFull with none taken"""
+        if n > len(self._free):
+            raise CacheFull("no free %s left (all %d are held)" % (self.what, self.n))
+        ids = self._free[len(self._free) - n:][::-1]
+        del self._free[len(self._free) - n:]
+        for i in ids:
+            if self._held[i]:
+                raise CacheError("%s %d was on the free list while held" % (self.what, i))
+            self._held[i] = True
+        return ids
+
     def give(self, i: int) -> None:
         if not (0 <= i < self.n):
             raise CacheError("%s %d does not exist (there are %d)" % (self.what, i, self.n))
@@ -93,19 +105,13 @@ class PageMap:
         row = self.rows[slot]
         first = self.n_blocks[slot]
         need = pages_for(new_len)
-        got: List[int] = []
-        try:
-            for b in range(first, need):
-                pg = self.pool.take()
-                got.append(b)
-                row[b] = pg
-                self.dirty.append((slot, b, pg))
-            self.n_blocks[slot] = max(first, need)
-        except CacheFull:
-            for b in got:
-                self.pool.give(row.pop(b))
-                self.dirty.append((slot, b, -1))
-            raise
+        if need <= first:
+            return
+        blocks = range(first, need)
+        pages = self.pool.take_many(need - first)            # (all or none)
+        row.update(zip(blocks, pages))
+        self.dirty.extend((slot, b, pg) for b, pg in zip(blocks, pages))
+        self.n_blocks[slot] = need
 
     def trim(self, slot: int, length: int) -> None:
         """give back the pages that no later query of this sequence can read (window groups only)"""

@@ -21,6 +21,7 @@ from typing import Dict, List, Optional, Sequence, Tuple
 import numpy as np
 import torch
 
+from ..kernels import lib as K
 from ..parts.base import KVNeed, StateNeed
 from .pages import PAGE, CacheError, FreeList, PageMap, pages_for
 
@@ -154,38 +155,42 @@ class SequenceCache:
 
     def flush(self) -> None:
         """bring the device page tables up to date (before a step's kernels are launched)"""
+        todo = []
         for g in self.groups:
             dirty = g.pages.take_dirty()
-            if not dirty:
-                continue
-            last: Dict[Tuple[int, int], int] = {}
-            for s, b, pg in dirty:
-                last[(s, b)] = pg
+            if dirty:
+                # (the last word on every place)
+                todo.append((g, {s * self.n_pages + b: pg for s, b, pg in dirty}))
+        if not todo:
+            return
+        if self.device.type != "cuda":
+            for g, last in todo:
+                idx = torch.tensor(list(last), dtype=torch.int64)
+                g.table.view(-1).index_copy_(0, idx, torch.tensor(list(last.values()), dtype=torch.int32))
+            return
+        # one launch a group that reads the places and the pages from pinned memory: a copy to the device, a conversion and a
+        # scatter issued one by one hold the host up for tens of microseconds before the step's first kernel
+        stage = self._stage(sum(len(last) for _, last in todo))
+        a = 0
+        for g, last in todo:
             n = len(last)
-            if self.device.type != "cuda":
-                idx = torch.tensor([s * self.n_pages + b for (s, b) in last], dtype=torch.int64)
-                val = torch.tensor(list(last.values()), dtype=torch.int32)
-                g.table.view(-1).index_copy_(0, idx, val)
-                continue
-            # one copy from pinned memory (places, then pages) instead of two from pageable memory, each of which
-            # would hold the host up for tens of microseconds before the step's first kernel
-            stage = self._stage(2 * n)
-            stage[:n] = torch.tensor([s * self.n_pages + b for (s, b) in last], dtype=torch.int64)
-            stage[n:2 * n] = torch.tensor(list(last.values()), dtype=torch.int64)
-            dev = stage[:2 * n].to(self.device, non_blocking=True)
-            self._stage_free.record()
-            g.table.view(-1).index_copy_(0, dev[:n], dev[n:].to(torch.int32))
+            self._stage_np[a:a + n, 0] = list(last)
+            self._stage_np[a:a + n, 1] = list(last.values())
+            K.table_set(g.table, stage[a:a + n], n)
+            a += n
+        self._stage_free.record()
 
     def _stage(self, n: int) -> torch.Tensor:
-        """pinned int64 staging memory of at least n elements, free to be written (the copy out of it that was issued
+        """pinned int32 staging memory of at least n pairs, free to be written (the copy out of it that was issued
         last has finished)"""
         buf = getattr(self, "_stage_buf", None)
         if buf is None:
             self._stage_free = torch.cuda.Event()
         else:
             self._stage_free.synchronize()
-        if buf is None or buf.numel() < n:
-            buf = self._stage_buf = torch.empty(max(256, 2 * n), dtype=torch.int64, pin_memory=True)
+        if buf is None or buf.shape[0] < n:
+            buf = self._stage_buf = torch.empty((max(256, 2 * n), 2), dtype=torch.int32, pin_memory=True)
+            self._stage_np = buf.numpy()
         return buf
 
     # ------------------------------------------------------------------ views for the parts

@@ -48,6 +48,23 @@ extern "C" int kb_embed(const void* table, int wdtype, const int* tok, float* x,
     KB_LAUNCH_RET();
 }
 
+// table[entries[i].x] = entries[i].y: the page table's new entries, read from the host's pinned memory. An ordinary launch:
+// kernels of the step before have finished, and the step's metadata copy behind it orders it before the step's kernels
+// (which read the table before their programmatic waits).
+__global__ void __launch_bounds__(256) k_table_set(int* table, long long size, const int2* entries, int n) {
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    if (i >= n) return;
+    const int2 e = entries[i];
+    if (e.x >= 0 && e.x < size) table[e.x] = e.y;
+}
+
+extern "C" int kb_table_set(int* table, long long size, const void* entries, int n, cudaStream_t st) {
+    if (n <= 0) return 0;
+    if ((uintptr_t)entries & 7) return (int)cudaErrorInvalidValue;
+    k_table_set<<<(n + 255) / 256, 256, 0, st>>>(table, size, (const int2*)entries, n);
+    KB_LAUNCH_RET();
+}
+
 // x[t] = table[tok[t]] * scale + pairs[bucket] + positions[pos[t]], in 32-bit. `pairs` (or null): a table over pairs of
 // neighbouring tokens, bucket = (previous token * mul_prev + token * mul_cur) mod buckets in 64-bit, and row `buckets` for a
 // sequence's first token. The previous token of the first row a sequence brings is what its last step left in `last`

@@ -7,6 +7,7 @@ tokens; ``rows`` are the packed row numbers, in the order of the entries and of 
 """
 from __future__ import annotations
 
+from array import array
 from dataclasses import dataclass
 from typing import List, Sequence, Tuple
 
@@ -97,7 +98,10 @@ def pack(entries: Sequence[StepEntry], length_before: Sequence[int], pad_rows_to
     kv_len = []
     for b, (e, n) in enumerate(zip(entries, q_len)):
         a = q_start[b]
-        tok[a:a + n] = e.tokens
+        try:
+            tok[a:a + n] = array("i", e.tokens)      # (a third faster than numpy's own walk over a tuple)
+        except TypeError:
+            tok[a:a + n] = e.tokens                  # (numbers that are no Python or numpy integers)
         pos[a:a + n] = np.arange(length_before[b], length_before[b] + n, dtype=np.int32)
         seq[a:a + n] = b
         kv_len.append(length_before[b] + n)

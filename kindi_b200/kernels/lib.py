@@ -40,6 +40,7 @@ _WKV = [c_int, c_void_p, c_void_p, c_void_p, c_int, c_longlong, c_int, c_void_p,
 
 _SIGS = {
     "kb_embed": [c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_float, c_void_p, c_void_p],
+    "kb_table_set": [c_void_p, c_longlong, c_void_p, c_int, c_void_p],
     "kb_embed_sum": [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                      c_longlong, c_longlong, c_longlong, c_int, c_int, c_void_p, c_int, c_int, c_int, c_float, c_void_p,
                      c_void_p],
@@ -330,6 +331,15 @@ def _need_cuda(*ts):
 
 
 # ----------------------------------------------------------------------------------------------- wrappers
+def table_set(table: torch.Tensor, entries: torch.Tensor, n: int) -> None:
+    """table.view(-1)[entries[2 i]] = entries[2 i + 1] for i < n (int32; ``entries`` in pinned host memory, which the kernel
+    reads in place and which may not change until it has run; the places are all different). Places outside the table
+    are left out. What follows on the stream starts after it"""
+    assert table.is_cuda and table.dtype == torch.int32 and table.is_contiguous()
+    assert entries.dtype == torch.int32 and entries.is_pinned() and entries.is_contiguous() and entries.numel() >= 2 * n
+    _check(load().kb_table_set(_p(table), table.numel(), _p(entries), n, _stream()), "table_set")
+
+
 def embed(table: torch.Tensor, tok: torch.Tensor, out: torch.Tensor, status: torch.Tensor,
           scale: float = 1.0) -> None:
     """out[t] (float32 [T, E]) = table[tok[t]] * scale"""

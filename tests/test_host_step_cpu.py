@@ -1,0 +1,44 @@
+"""The host's side of a step: pages handed out many at a time are those that one at a time would have been, a full pool takes
+none, and token ids in any numeric form are packed alike."""
+import numpy as np
+import pytest
+
+from kindi_b200.cache.pages import CacheFull, FreeList, PageMap
+from kindi_b200.engine.batch import StepEntry, pack
+
+
+def test_many_ids_at_a_time_are_the_ones_taken_one_by_one():
+    a, b = FreeList(9, "page"), FreeList(9, "page")
+    for f in (a, b):
+        for i in [f.take() for _ in range(6)][1::2]:
+            f.give(i)
+    assert a.take_many(4) == [b.take() for _ in range(4)]
+    a.check()
+    left = a.n_free
+    with pytest.raises(CacheFull):
+        a.take_many(left + 1)
+    assert a.n_free == left
+    assert a.take_many(0) == []
+    a.check()
+
+
+def test_a_full_pool_leaves_a_sequence_as_it_was():
+    pm = PageMap(n_pages=3, n_slots=2)
+    pm.ensure(0, 65)
+    pm.take_dirty()
+    with pytest.raises(CacheFull):
+        pm.ensure(1, 129)
+    assert pm.take_dirty() == [] and pm.rows[1] == {} and pm.n_blocks[1] == 0
+    pm.ensure(0, 10)                                   # nothing new
+    assert pm.take_dirty() == []
+    pm.ensure(1, 64)
+    pm.check()
+
+
+@pytest.mark.parametrize("form", [tuple, list, lambda t: np.array(t, dtype=np.int64), lambda t: tuple(np.int32(x) for x in t),
+                                  lambda t: tuple(float(x) for x in t)])
+def test_token_ids_in_any_form(form):
+    toks = (3, 0, 70000, 9)
+    ps = pack([StepEntry(0, form(toks), (3,)), StepEntry(1, form((5, 6)), ())], [0, 2])
+    a, n = ps.off["tok"]
+    assert ps.meta[a:a + n].tolist() == [3, 0, 70000, 9, 5, 6]

@@ -648,3 +648,20 @@ def test_norm_of_rows_shared_by_warps(K, kind, T, E, planes, scaled):
         assert _rel(x, v) < 1e-6
         # one bf16 rounding of the result, 2^-9 of a value
         assert float(((y.double() - want).abs() / (want.abs() + 1e-2)).max()) < 2 ** -8
+
+
+def test_page_table_entries_from_pinned_memory(K):
+    table = torch.full((3, 700), -1, dtype=torch.int32, device="cuda")
+    want = table.clone()
+    for n in (1, 255, 257, 900):
+        e = torch.empty((max(n, 300), 2), dtype=torch.int32, pin_memory=True)
+        at = torch.randperm(table.numel())[:n].int()
+        e[:n, 0], e[:n, 1] = at, torch.arange(n, dtype=torch.int32) + n
+        if n == 257:
+            e[5, 0], e[6, 0] = table.numel(), -1           # places outside the table are left out
+        for i, v in e[:n].tolist():
+            if 0 <= i < table.numel():
+                want.view(-1)[i] = v
+        K.table_set(table, e, n)
+        torch.cuda.synchronize()
+        assert torch.equal(table, want)
