@@ -38,10 +38,43 @@ __global__ void k_embed(const TW* __restrict__ table, const int* __restrict__ to
     }
 }
 
+// The same row eight elements a thread (16 or 32 bytes in, 32 out, the same product): widths that are multiples of 8 with
+// aligned tables. An element a thread and pass made a row's loads wait for one another: eight rows of 2560 7.3 -> 2 us,
+// 2048 rows 12.1 -> 8.7 us, 8171 of 5120 84 -> 66 us (3.8 TB/s).
+template <typename TW>
+__global__ void __launch_bounds__(256) k_embed8(const TW* __restrict__ table, const int* __restrict__ tok, float* __restrict__ x,
+                                                int E, int vocab, float scale, int* status) {
+    kb_pdl_launch();
+    kb_pdl_wait();
+    const int t = blockIdx.x, c = (blockIdx.y * 256 + threadIdx.x) * 8;
+    if (c >= E) return;
+    const int id = tok[t];
+    float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    if (id < 0 || id >= vocab) {
+        if (c == 0) atomicOr(status, KB_ST_BAD_TOKEN);
+    } else {
+        const TW* p = table + (size_t)id * E + c;
+        TW raw[8];
+        *(uint4*)raw = *(const uint4*)p;
+        if (sizeof(TW) == 4) *(uint4*)(raw + 4) = *(const uint4*)(p + 4);
+#pragma unroll
+        for (int i = 0; i < 8; i++) v[i] = scale == 1.0f ? kb_to_f<TW>(raw[i]) : kb_to_f<TW>(raw[i]) * scale;
+    }
+    float4* o = (float4*)(x + (size_t)t * E + c);
+    o[0] = make_float4(v[0], v[1], v[2], v[3]);
+    o[1] = make_float4(v[4], v[5], v[6], v[7]);
+}
+
 // x[t] = table[tok[t]] * scale (scale 1: the row as stored, the reference's embedding: kindi/nbq.cu:472-487)
 extern "C" int kb_embed(const void* table, int wdtype, const int* tok, float* x, int T, int E, int vocab,
                         float scale, int* status, cudaStream_t st) {
     if (T <= 0) return 0;
+    if (E % 8 == 0 && ((uintptr_t)table & 15) == 0 && ((uintptr_t)x & 15) == 0) {
+        const dim3 grid(T, (E / 8 + 255) / 256);
+        if (wdtype == KB_F32) kb_launch(k_embed8<float>, grid, 256, 0, st, (const float*)table, tok, x, E, vocab, scale, status);
+        else kb_launch(k_embed8<bf16>, grid, 256, 0, st, (const bf16*)table, tok, x, E, vocab, scale, status);
+        KB_LAUNCH_RET();
+    }
     if (wdtype == KB_F32)
         kb_launch(k_embed<float>, T, 256, 0, st, (const float*)table, tok, x, E, vocab, scale, status);
     else kb_launch(k_embed<bf16>, T, 256, 0, st, (const bf16*)table, tok, x, E, vocab, scale, status);
