@@ -78,10 +78,6 @@ class SequenceCache:
             if states:
                 self.state[i] = [torch.zeros((self.n_slots,) + tuple(st.shape), dtype=torch.float32,
                                              device=self.device) for st in states]
-        # how many of a sequence's parts have arrived, per sequence of a step and key/value head: the decode attention's parts
-        # merge themselves and leave zeros (a step's kernels run one after the other, so one array serves all layers)
-        heads = max((n.n_kv_heads for n in by_need), default=0)
-        self.arrivals = torch.zeros(self.n_slots * heads, dtype=torch.int32, device=self.device)
         for need, entries in by_need.items():
             n_pool = self.group_pages(need, self.n_pages, self.n_slots, max_step_tokens)
             pool = torch.zeros((len(entries), n_pool, need.planes, need.n_kv_heads, PAGE, need.head_dim), dtype=dtype,

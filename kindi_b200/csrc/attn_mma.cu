@@ -77,64 +77,13 @@ __device__ __forceinline__ void at_ld_sum(const float* const (&p)[NS], const boo
                 }
     }
 }
-// Sequences of unequal lengths that nearly fill the SMs: the longest are cut into parts. A CTA gets through about 1.1 pages a
-// microsecond, so a step whose (sequence, head) pairs have a CTA each lasts as long as its longest sequence: 48 sequences of
-// 203 to 6007 positions x 4 heads, 70 us a layer for 305 MB. A part holds at most P pages, P being what a CTA gets through
-// while the memory delivers all of them (a 180th of the sum), or more when the parts would not fit one wave (`items` CTAs per
-// key/value head). Equal lengths stay whole. Item i of the list of all parts, sequence after sequence, is CTA i's; each
-// CTA's first warp finds its own from the step's lengths, before the wait on the preceding kernel: 62.5 us.
-// (Dealt out the same way in steps of few sequences, whose splits fill the SMs anyway, with the merge kernel finding its
-// parts too: 2.67 -> 2.83 ms a step of eight sequences of 8192.)
-struct AtDeal {
-    int items;                  // 0: gridDim.x splits for every sequence
-    int B;
-    int* arrivals;              // [B][nkv], zeros between launches: the last part to finish merges its sequence's
-};
-#define AT_DEAL_SHARE 180
-__device__ __forceinline__ int at_pages(int kvl) { return (kvl + KB_PAGE - 1) / KB_PAGE; }
-// (sequence, part, its sequence's parts, the first one's item) of an item; sequence -1: more items than parts. Whole warp.
-__device__ __forceinline__ int4 at_deal(const AtDeal& d, const int* __restrict__ kv_len, int nkv, int item, int lane) {
-    int most = 1, sum = 0;
-    for (int b = lane; b < d.B; b += 32) {
-        const int n = at_pages(kv_len[b]);
-        most = max(most, n);
-        sum += n;
-    }
-    most = __reduce_max_sync(0xffffffffu, most);
-    sum = __reduce_add_sync(0xffffffffu, sum);
-    int P = min(most, (int)(((long long)sum * nkv + AT_DEAL_SHARE - 1) / AT_DEAL_SHARE));
-    for (; P < most; P += 1 + P / 16) {
-        int parts = 0;
-        for (int b = lane; b < d.B; b += 32) parts += (at_pages(kv_len[b]) + P - 1) / P;
-        if (__reduce_add_sync(0xffffffffu, parts) <= d.items) break;
-    }
-    int before = 0;
-    for (int b0 = 0; b0 < d.B; b0 += 32) {
-        const int b = b0 + lane;
-        const int n = b < d.B ? (at_pages(kv_len[b]) + P - 1) / P : 0;
-        int up = n;                                    // parts up to and with this lane's sequence
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(0xffffffffu, up, o);
-            if (lane >= o) up += v;
-        }
-        const unsigned m = __ballot_sync(0xffffffffu, item >= before + up - n && item < before + up);
-        if (m) {
-            const int l = __ffs(m) - 1;
-            const int nn = __shfl_sync(0xffffffffu, n, l), first = before + __shfl_sync(0xffffffffu, up, l) - nn;
-            return make_int4(b0 + l, item - first, nn, first);
-        }
-        before += __shfl_sync(0xffffffffu, up, 31);
-    }
-    return make_int4(-1, 0, 0, 0);
-}
 template <int HD, bool DEC, bool ROPE = false>
 __global__ void __launch_bounds__(AT_THREADS, 2) k_attn_mma(const __grid_constant__ CUtensorMap kvmap,
-        const bf16* KB_STEP_DATA q, int ldq, bf16* __restrict__ out, int ldo, float* KB_STEP_DATA part_o,
-        float* KB_STEP_DATA part_ml, const int* __restrict__ slot, const int* __restrict__ q_start,
+        const bf16* KB_STEP_DATA q, int ldq, bf16* __restrict__ out, int ldo, float* __restrict__ part_o,
+        float* __restrict__ part_ml, const int* __restrict__ slot, const int* __restrict__ q_start,
         const int* __restrict__ kv_len, int nh, int nkv, int G, float scale_log2e, int window,
         const int* __restrict__ table, int table_stride, int n_pages, int* status, AtRopeIn rp, int keep_first,
-        const float* __restrict__ sink, int chunk, const __grid_constant__ KbCap cap, AtDeal deal) {
+        const float* __restrict__ sink, int chunk, const __grid_constant__ KbCap cap) {
     static_assert(!ROPE || DEC, "rotation inside the kernel: decode form only");
     constexpr int AT_STAGES = DEC ? 3 : 2;      // pages in flight (two CTAs fit an SM in both forms)
     constexpr int KT = HD / 16;                 // k-steps of Q K^T
@@ -151,25 +100,7 @@ __global__ void __launch_bounds__(AT_THREADS, 2) k_attn_mma(const __grid_constan
     // writes the same values
     bf16* qs = (bf16*)(smem + AT_STAGES * STAGE_BYTES + 2 * AT_STAGES * 8 + 16);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int hk = blockIdx.y;
-    int b = blockIdx.z, n_splits = gridDim.x, split = blockIdx.x, item0 = 0;
-    if (DEC && !ROPE && deal.items > 0) {
-        __shared__ int4 s_part;
-        if (warp == 0) {
-            const int4 v = at_deal(deal, kv_len, nkv, blockIdx.x, lane);
-            if (lane == 0) s_part = v;
-        }
-        __syncthreads();
-        const int4 part = s_part;
-        if (part.x < 0) {                            // more CTAs than parts
-            kb_pdl_launch_now();
-            return;
-        }
-        b = part.x;
-        split = part.y;
-        n_splits = part.z;
-        item0 = part.w;
-    }
+    const int b = blockIdx.z, hk = blockIdx.y;
     // The step's metadata (lengths, slots, page table) was written before the step's first kernel, and the pages of
     // older positions by earlier steps. In the decode form only Q and the page of the newest position come from the
     // kernel just before this one, so each thread waits for that kernel where it first needs them.
@@ -188,8 +119,8 @@ __global__ void __launch_bounds__(AT_THREADS, 2) k_attn_mma(const __grid_constan
         pg_first = lo / KB_PAGE;
         n_keep = min((keep_first + KB_PAGE - 1) / KB_PAGE, pg_first);
         const int total = n_keep + last - pg_first + 1;
-        const int per = (total + n_splits - 1) / n_splits;                       // ceil(pages / splits)
-        it_lo = split * per;
+        const int per = (total + (int)gridDim.x - 1) / (int)gridDim.x;           // ceil(pages / splits)
+        it_lo = (int)blockIdx.x * per;
         n_iter = min(total, it_lo + per) - it_lo;                                // may be <= 0 for an empty split
     } else {
         const int n_tiles = (n_rows + AT_ROWS - 1) / AT_ROWS;
@@ -523,6 +454,7 @@ __global__ void __launch_bounds__(AT_THREADS, 2) k_attn_mma(const __grid_constan
         }
     }
     __syncthreads();
+    const int n_splits = gridDim.x, split = blockIdx.x;
     for (int e = threadIdx.x; e < G * HD; e += AT_THREADS) {
         const int r = e / HD, d = e % HD;
         float M = -INFINITY;
@@ -541,40 +473,13 @@ __global__ void __launch_bounds__(AT_THREADS, 2) k_attn_mma(const __grid_constan
             if (sink != nullptr) lv += exp2f(sink[h] * 1.4426950408889634f - U);
             out[(size_t)qs0 * ldo + (size_t)h * HD + d] = __float2bfloat16_rn(lv > 0.0f ? ov / lv : 0.0f);
         } else {
-            const size_t pi = !ROPE && deal.items > 0 ? (size_t)(item0 + split) * nh + h : ((size_t)b * nh + h) * n_splits + split;
+            const size_t pi = ((size_t)b * nh + h) * n_splits + split;
             part_o[pi * HD + d] = ov;
             if (d == 0) {
                 part_ml[pi * 2] = M;
                 part_ml[pi * 2 + 1] = lv;
             }
         }
-    }
-    if (ROPE || deal.items == 0 || n_splits == 1) return;
-    // The last of the sequence's parts to get here adds them all, in their order. The counter goes back to zero by itself
-    // (atomicInc wraps after n_splits arrivals). A part more or less is rare enough in such steps that a kernel of its own
-    // for the merge, which every step would wait for, costs more.
-    __shared__ int s_last;
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0)
-        s_last = atomicInc((unsigned*)deal.arrivals + (size_t)b * nkv + hk, (unsigned)n_splits - 1u) == (unsigned)n_splits - 1u;
-    __syncthreads();
-    if (!s_last) return;
-    __threadfence();
-    for (int e = threadIdx.x; e < G * HD; e += AT_THREADS) {
-        const int h = hk * G + e / HD, d = e % HD;
-        float M = -INFINITY;
-        for (int s = 0; s < n_splits; s++) M = fmaxf(M, __ldcg(part_ml + ((size_t)(item0 + s) * nh + h) * 2));
-        const float U = M == -INFINITY ? 0.0f : M;
-        float ov = 0.0f, lv = 0.0f;
-        for (int s = 0; s < n_splits; s++) {
-            const size_t pi = (size_t)(item0 + s) * nh + h;
-            const float f = exp2f(__ldcg(part_ml + pi * 2) - U);
-            ov = fmaf(f, __ldcg(part_o + pi * HD + d), ov);
-            lv = fmaf(f, __ldcg(part_ml + pi * 2 + 1), lv);
-        }
-        if (sink != nullptr) lv += exp2f(sink[h] * 1.4426950408889634f - U);
-        out[(size_t)qs0 * ldo + (size_t)h * HD + d] = __float2bfloat16_rn(lv > 0.0f ? ov / lv : 0.0f);
     }
 }
 
@@ -589,8 +494,8 @@ __global__ void k_attn_merge(const float* KB_STEP_DATA part_o, const float* KB_S
     __shared__ float so[4][256];
     __shared__ float s_sink;                      // the sink's share of the denominator, relative to M
     kb_pdl_launch();
-    const int h = blockIdx.x, b = blockIdx.y;
     kb_pdl_wait();
+    const int h = blockIdx.x, b = blockIdx.y;
     const size_t base = ((size_t)b * nh + h) * n_splits;
     if (threadIdx.x < 32) {
         float m0 = threadIdx.x < n_splits ? part_ml[(base + threadIdx.x) * 2] : -INFINITY;
@@ -648,7 +553,7 @@ static int launch_attn(const CUtensorMap& map, const void* q, int ldq, void* out
                        float* part_ml, const int* slot, const int* q_start, const int* kv_len, int B, int nh, int nkv,
                        float scale, int window, const int* table, int table_stride, int n_pages, int grid_x,
                        int* status, cudaStream_t st, AtRopeIn rp = AtRopeIn(), int keep_first = 0,
-                       const float* sink = nullptr, int chunk = 0, const KbCap& cap = KbCap(), const AtDeal& deal = AtDeal()) {
+                       const float* sink = nullptr, int chunk = 0, const KbCap& cap = KbCap()) {
     auto kern = k_attn_mma<HD, DEC, ROPE>;
     int sm = attn_smem_bytes<HD, DEC>();
     constexpr int ALONE = 118 * 1024;   // more than half of an SM's shared memory: a CTA that asks for it has the SM to itself
@@ -660,11 +565,11 @@ static int launch_attn(const CUtensorMap& map, const void* q, int ldq, void* out
     // A decode step with no more CTAs than SMs: every CTA gets an SM of its own. Placed while the kernel before still
     // holds some SMs, the CTAs were otherwise put two by two on the free ones, where two position streams share
     // what one SM can take in (32 sequences x 4 heads at context 8192: 4.97 -> 4.68 ms a step).
-    if (DEC && (long long)grid_x * nkv * (deal.items > 0 ? 1 : B) <= kb_sm_count_attn() && sm < ALONE) sm = ALONE;
-    dim3 grid(grid_x, nkv, deal.items > 0 ? 1 : B);
+    if (DEC && (long long)grid_x * nkv * B <= kb_sm_count_attn() && sm < ALONE) sm = ALONE;
+    dim3 grid(grid_x, nkv, B);
     kb_launch(kern, grid, AT_THREADS, sm, st, map, (const bf16*)q, ldq, (bf16*)out, ldo, part_o, part_ml, slot, q_start,
                                        kv_len, nh, nkv, nh / nkv, scale * 1.4426950408889634f, window, table,
-                                       table_stride, n_pages, status, rp, keep_first, sink, chunk, cap, deal);
+                                       table_stride, n_pages, status, rp, keep_first, sink, chunk, cap);
     return (int)cudaGetLastError();
 }
 
@@ -675,21 +580,12 @@ extern "C" int kb_attn_mma(const void* q, int ldq, void* out, int ldo, float* pa
                            const int* slot, const int* q_start, const int* kv_len, int B, int nh, int nkv, int hd,
                            float scale, int window, void* pool, const int* table, int table_stride, int n_pages,
                            int decode, int grid_x, int* status, cudaStream_t st, int keep_first, const float* sink,
-                           int chunk, const float* cap, int deal_items = 0, int* arrivals = nullptr) {
-    // deal_items > 0 (decode, every position seen: no window, no chunk): the longest sequences' pages dealt out over up to that
-    // many parts per key/value head, at least B, which merge themselves; part_o [deal_items][nh][hd] and part_ml
-    // [deal_items][nh][2] are scratch, arrivals (int [B][nkv]) is zero and zero again after the call
+                           int chunk, const float* cap) {
     // sink (float [nh] or null): exp(sink[h]) joins head h's softmax denominator, once (with position splits: in the
     // merge). chunk > 0: a row sees its own chunk of that many positions. cap: see kb_cap_of
     if (B <= 0 || grid_x <= 0) return 0;
     if (window <= 0 || keep_first < 0) keep_first = 0;
-    if (deal_items > 0) {
-        if (!decode || window > 0 || chunk > 0 || deal_items < B || !part_o || !part_ml || !arrivals) return (int)cudaErrorInvalidValue;
-        grid_x = deal_items;
-    } else if (decode && grid_x > 64) {
-        return (int)cudaErrorInvalidValue;
-    }
-    const AtDeal deal{deal_items, B, arrivals};
+    if (decode && grid_x > 64) return (int)cudaErrorInvalidValue;
     if ((hd != 64 && hd != 128) || nkv <= 0 || nh % nkv) return (int)cudaErrorInvalidValue;
     if (decode && nh / nkv > 16) return (int)cudaErrorInvalidValue;
     if ((ldq % 8) || (ldo % 2) || ((uintptr_t)q & 15)) return (int)cudaErrorInvalidValue;
@@ -699,7 +595,7 @@ extern "C" int kb_attn_mma(const void* q, int ldq, void* out, int ldo, float* pa
 #define AT_GO(HD, DEC)                                                                                          \
     rc = launch_attn<HD, DEC>(map, q, ldq, out, ldo, part_o, part_ml, slot, q_start, kv_len, B, nh, nkv, scale, \
                               window, table, table_stride, n_pages, grid_x, status, st, AtRopeIn(), keep_first, sink, \
-                              chunk, kb_cap_of(cap), deal)
+                              chunk, kb_cap_of(cap))
     if (hd == 128) {
         if (decode) AT_GO(128, true); else AT_GO(128, false);
     } else {
@@ -707,7 +603,7 @@ extern "C" int kb_attn_mma(const void* q, int ldq, void* out, int ldo, float* pa
     }
 #undef AT_GO
     if (rc) return rc;
-    if (decode && grid_x > 1 && deal_items == 0) {
+    if (decode && grid_x > 1) {
         dim3 grid(nh, B);
         kb_launch(k_attn_merge, grid, 4 * hd, 0, st, part_o, part_ml, grid_x, (bf16*)out, ldo, q_start, nh, hd, sink);
         return (int)cudaGetLastError();

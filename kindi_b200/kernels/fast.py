@@ -290,12 +290,10 @@ def attention_bf16(ctx, q, out, nh, nkv, hd, scale, window, pool, table, n_pages
                 cap=cap.host if cap is not None else None)
     if ctx.decode and g <= 16:
         splits = decode_splits(ctx, nkv)
-        deal = decode_deal(ctx, nkv) if splits == 1 and not window and chunk == 0 else 0
         if chunk > 0:
             splits = min(splits, -(-chunk // K.PAGE) + 1)          # (no more splits than pages a chunk can touch)
         K.attn_mma(q, out, ctx.slot, ctx.q_start, ctx.kv_len, ctx.B, nh, nkv, hd, scale, window, pool, table,
-                   n_pages, decode=True, grid_x=splits, deal=deal,
-                   arrivals=ctx.cache.arrivals if deal else None, **more)
+                   n_pages, decode=True, grid_x=splits, **more)
         return 1
     # (in a recording ctx.max_q is the most rows a sequence can bring: the grid then has tiles to spare, which leave)
     if g <= 128 and out.stride(0) % 8 == 0 and out.data_ptr() % 16 == 0:
@@ -318,19 +316,6 @@ def decode_splits(ctx, nkv: int) -> int:
     contexts and faster at short ones (32 sequences x 4 heads, 8 layers: 0.732 against 0.779 ms at context 512)"""
     s = 2 * N_SM // (ctx.B * nkv)
     return 1 if s <= 2 else min(64, s)
-
-
-def decode_deal(ctx, nkv: int) -> int:
-    """parts per key/value head over which the longest sequences of a decode step may be cut, or 0: no sequence is cut other
-    than by ``decode_splits``. Where the (sequence, head) pairs fill the SMs more than once, the longest sequences' pages
-    then run beside the others' instead of alone at the end (48 sequences of 203 to 6007 positions x 4 heads, eight layers:
-    1080 -> 1017 us); sequences of equal lengths stay whole. With no more pairs than SMs every pair has an SM to itself, which is worth more
-    (see launch_attn)"""
-    pairs = ctx.B * nkv
-    have = getattr(ctx.cache, "arrivals", None)
-    if N_SM < pairs <= 2 * N_SM and have is not None and have.numel() >= pairs:
-        return 2 * N_SM // nkv
-    return 0
 
 
 def attention_decode_rope(ctx, qkv, out, nh, nkv, hd, scale, window, inv_freq, rotary_dim, pool, store, table,

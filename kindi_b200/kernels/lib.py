@@ -142,7 +142,7 @@ _SIGS = {
                               c_void_p, c_void_p, c_void_p, c_int, c_float, c_float],
     "kb_attn_mma": [c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int,
                     c_int, c_int, c_float, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
-                    c_int, c_void_p, c_int, c_void_p, c_int, c_void_p],
+                    c_int, c_void_p, c_int, c_void_p],
     "kb_attn_decode_rope": [c_void_p, c_int, c_longlong, c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p,
                             c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p, c_int, c_void_p,
                             c_int, c_int, c_int, c_void_p, c_void_p],
@@ -1030,29 +1030,26 @@ def gemm_tc_splits(K: int, wanted: int) -> int:
 def attn_mma(q: torch.Tensor, out: torch.Tensor, slot, q_start, kv_len, B: int, nh: int, nkv: int, hd: int,
              scale: float, window: int, pool: torch.Tensor, table: torch.Tensor, n_pages: int, *, decode: bool,
              grid_x: int, status: torch.Tensor, keep_first: int = 0, sink: Optional[torch.Tensor] = None,
-             chunk: int = 0, cap=None, deal: int = 0, arrivals: Optional[torch.Tensor] = None) -> None:
+             chunk: int = 0, cap=None) -> None:
     """tensor-core attention over the cache (bf16, head size 64 or 128). decode: one row per sequence, grid_x =
     position splits; else grid_x = ceil(most rows of a sequence * (nh / nkv) / 64). ``keep_first``: with a window,
     the sequence's first positions that stay visible. ``sink`` (float32 [nh]): exp(sink[h]) joins head h's softmax
     denominator. ``chunk`` > 0: a row sees the positions of its own chunk. ``cap``: the ten host floats of a score cap
-    (``attention.ScoreCap.host``). ``deal`` (decode without window or chunk; at least B): the longest sequences' pages are
-    dealt out over up to that many parts per key/value head, whatever grid_x, with ``arrivals`` (int32, B nkv zeros, which it
-    leaves as zeros)"""
-    _need_cuda(q, out, pool, table, sink, arrivals)
-    assert (arrivals is None and not deal) or (arrivals.dtype == torch.int32 and arrivals.is_contiguous() and arrivals.numel() >= B * nkv)
+    (``attention.ScoreCap.host``)"""
+    _need_cuda(q, out, pool, table, sink)
     if sink is not None:
         assert sink.dtype == torch.float32 and sink.is_contiguous() and sink.numel() == nh
     assert q.dtype == out.dtype == pool.dtype == torch.bfloat16 and q.stride(1) == 1 and out.stride(1) == 1
     assert pool.is_contiguous()
     part_o = part_ml = None
-    if decode and (grid_x > 1 or deal):
-        part_o = torch.empty((deal or B * grid_x, nh, hd), dtype=torch.float32, device=q.device)
-        part_ml = torch.empty((deal or B * grid_x, nh, 2), dtype=torch.float32, device=q.device)
+    if decode and grid_x > 1:
+        part_o = torch.empty((B, nh, grid_x, hd), dtype=torch.float32, device=q.device)
+        part_ml = torch.empty((B, nh, grid_x, 2), dtype=torch.float32, device=q.device)
     _check(load().kb_attn_mma(_p(q), q.stride(0), _p(out), out.stride(0), _p(part_o), _p(part_ml), _p(slot),
                               _p(q_start), _p(kv_len), B, nh, nkv, hd, float(scale), int(window), _p(pool), _p(table),
                               table.stride(0), n_pages, 1 if decode else 0, grid_x, _p(status), _stream(),
-                              int(keep_first), _p(sink), int(chunk), cap, int(deal), _p(arrivals)), "attn_mma")
-    if decode and grid_x > 1 and not deal:
+                              int(keep_first), _p(sink), int(chunk), cap), "attn_mma")
+    if decode and grid_x > 1:
         add_launches(1)         # the merge of the position splits
 
 

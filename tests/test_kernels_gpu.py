@@ -665,55 +665,3 @@ def test_page_table_entries_from_pinned_memory(K):
         K.table_set(table, e, n)
         torch.cuda.synchronize()
         assert torch.equal(table, want)
-
-
-@pytest.mark.parametrize("kv_lens,deal", [
-    ([1], 1), ([700], 9), ([64, 65, 1, 1300, 129], 5), ([64, 65, 1, 1300, 129], 12), ([640] * 6, 24), ([640] * 180, 200),
-    ([1 + 37 * (i * 7 % 41) for i in range(41)], 60), ([2500] + [3] * 70, 74)])
-@pytest.mark.parametrize("nh,nkv,hd", [(20, 4, 128), (3, 1, 64)])
-def test_attention_decode_with_pages_dealt_out(K, kv_lens, deal, nh, nkv, hd):
-    """parts of unequal sequences that merge themselves, as few parts as sequences and more parts than pages; equal sequences
-    stay whole; the counters are zero again, also when the call is repeated"""
-    B = len(kv_lens)
-    pool, table, dense, slots, n_pages = _make_cache(kv_lens, nkv, hd, torch.bfloat16, seed=B + deal)
-    g = torch.Generator(device="cpu").manual_seed(B)
-    q = torch.randn(B, nh, hd, generator=g).to(torch.bfloat16)
-    sink = torch.randn(nh, generator=g).cuda()
-    dev = lambda x: torch.tensor(x, dtype=torch.int32).cuda()      # noqa: E731
-    scale = 1.0 / math.sqrt(hd)
-    arrivals, st = torch.zeros(B * nkv + 3, dtype=torch.int32, device="cuda"), _status()
-
-    def go(splits=1, **more):
-        out = torch.full((B, nh * hd), float("nan"), dtype=torch.bfloat16, device="cuda")
-        K.attn_mma(q.reshape(B, nh * hd).cuda(), out, slots, dev(list(range(B + 1))), dev(kv_lens), B, nh, nkv, hd, scale, 0,
-                   pool, table, n_pages, decode=True, grid_x=splits, status=st, **more)
-        assert int(st.item()) == 0 and int(arrivals.abs().sum()) == 0
-        return out
-    for with_sink in (None, sink):
-        plain = go(sink=with_sink)
-        for got in (go(deal=deal, arrivals=arrivals, sink=with_sink), go(deal=deal, arrivals=arrivals, sink=with_sink)):
-            # two orders of one 32-bit sum, each rounded to bf16 once
-            assert float((got.float() - plain.float()).abs().max() / plain.float().abs().max()) < 2 ** -7
-    if len(set(kv_lens)) == 1 and B * nkv >= 180:
-        assert torch.equal(go(deal=deal, arrivals=arrivals), go())          # equal sequences stay whole
-    ref = torch.cat([_attn_ref(q[b:b + 1].float(), dense[b][0].float(), dense[b][1].float(), [n - 1], scale, 0)
-                     for b, n in enumerate(kv_lens)])
-    assert float((go(deal=deal, arrivals=arrivals).double().cpu().reshape(B, nh, hd) - ref).abs().max() / ref.abs().max()) < 1e-2
-
-
-@pytest.mark.parametrize("E", [8, 40, 2048, 2056, 2060, 4104])
-@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("scale", [1.0, 0.37])
-def test_embedding_rows_of_every_width(K, E, dtype, scale):
-    """rows in pieces of eight and rows that are not, tables that are aligned and one that is not, ids outside the table"""
-    g = torch.Generator(device="cuda").manual_seed(E)
-    store = torch.randn(50 * E + 8, device="cuda", generator=g).to(dtype)
-    tok = torch.tensor([0, 49, 7, 50, -1, 3, 2 ** 30], dtype=torch.int32, device="cuda")
-    for at in (0, 1):
-        table = store[at:at + 50 * E].view(50, E)
-        out, st = torch.full((7, E), 9.0, device="cuda"), _status()
-        K.embed(table, tok, out, st, scale)
-        want = torch.zeros(7, E, device="cuda")
-        ok = (tok >= 0) & (tok < 50)
-        want[ok] = table[tok[ok].long()].float() * torch.tensor(scale, device="cuda")
-        assert torch.equal(out, want) and int(st.item()) == K.ST_BAD_TOKEN

@@ -111,6 +111,32 @@ def test_wide_decode_batch_at_layer_sizes(tmp_path):
     _compare(tiny.collect(out, steps, vocab), reqs, want, TOL["bfloat16"], "layer-sized")
 
 
+@pytest.mark.parametrize("n_seq", [40, 64])
+def test_a_wide_decode_steps_row_does_not_depend_on_its_neighbours_lengths(tmp_path, n_seq):
+    """more (sequence, key/value head) pairs than SMs: a sequence's logits are the same bits whether the others hold few
+    positions or many, in unrecorded and in recorded steps of one row count"""
+    from kindi_b200.engine.batch import StepEntry
+    from kindi_b200.engine.engine import Engine
+    cfg = dict(LONG, hidden_size=256, num_attention_heads=8, num_key_value_heads=4, head_dim=64)
+    eng = Engine(tiny.make_needle_model(tmp_path, cfg, seed=61, name="wide"), ctx=n_seq * 1100 + 2000, max_batch=n_seq)
+    rng = random.Random(5)
+    vocab = cfg["vocab_size"]
+    toks = [tuple(rng.randrange(3, vocab) for _ in range(1301)) for _ in range(n_seq)]
+    got = []
+    for others in (5, 130, 1000):
+        slots = [eng.alloc() for _ in range(n_seq)]
+        lens = [1300] + [others] * (n_seq - 1)
+        for s, t, n in zip(slots, toks, lens):
+            eng.step([StepEntry(s, t[:n], ())])
+        rows = [eng.step([StepEntry(s, (t[i],), (0,)) for s, t in zip(slots, toks)])[0].clone() for i in range(5)]
+        got.append(torch.stack(rows).cpu())
+        eng.check_status()
+        for s in slots:
+            eng.free(s)
+    assert eng.graph_replays > 0
+    assert torch.equal(got[0], got[1]) and torch.equal(got[0], got[2])
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 def test_context_of_more_than_8192_positions(tmp_path, dtype):
     """one request of 8,230 tokens: the prompt goes through pieces of max_step_tokens, the last 32 tokens one by one,
