@@ -265,6 +265,7 @@ __global__ void __launch_bounds__(256, 2) k_decay_out(const TIN* KB_STEP_DATA in
     for (int us = 0; us <= u; us++) {
         const bool diag = us == u;
         const int ns = min(DQ_T, nc_rows - us * DQ_T);
+        float probe = 0.0f;                           // stays zero while this thread's values are finite
         if (us == 0 && raw) {
             uint4 rk[DQ_T * D / 8 / 256], rv[DQ_T * DQ_E / 8 / 256];
 #pragma unroll
@@ -293,8 +294,10 @@ __global__ void __launch_bounds__(256, 2) k_decay_out(const TIN* KB_STEP_DATA in
 #pragma unroll
                 for (int y = 0; y < 4; y++) {
                     const float2 f = __bfloat1622float2(h2[y]);
-                    vt[(j + 2 * y) * DQ_LV + t] = dq_silu(f.x);
-                    vt[(j + 2 * y + 1) * DQ_LV + t] = dq_silu(f.y);
+                    const float v0 = dq_silu(f.x), v1 = dq_silu(f.y);
+                    vt[(j + 2 * y) * DQ_LV + t] = v0;
+                    vt[(j + 2 * y + 1) * DQ_LV + t] = v1;
+                    probe = fmaf(v0, 0.0f, fmaf(v1, 0.0f, probe));
                 }
             }
         } else {
@@ -307,11 +310,14 @@ __global__ void __launch_bounds__(256, 2) k_decay_out(const TIN* KB_STEP_DATA in
             // (neighbouring lanes take neighbouring tokens, so that the transposed stores fall into different banks)
             dq_stage<TIN, DQ_E, true>(in, a.n_planes, a.plane_stride, a.ld_in, rc + us * DQ_T, ns, ov, a.dv - e0, a.vec_v,
                                       [&](int t, int j, const float* v) {
-    #pragma unroll
-                                          for (int x = 0; x < 8; x++) vt[(j + x) * DQ_LV + t] = v[x];
+#pragma unroll
+                                          for (int x = 0; x < 8; x++) {
+                                              vt[(j + x) * DQ_LV + t] = v[x];
+                                              probe = fmaf(v[x], 0.0f, probe);
+                                          }
                                       });
         }
-        __syncthreads();
+        const bool odd = __syncthreads_or(!(probe == 0.0f));
         float s4[4][4];
 #pragma unroll
         for (int i = 0; i < 4; i++)
@@ -327,6 +333,25 @@ __global__ void __launch_bounds__(256, 2) k_decay_out(const TIN* KB_STEP_DATA in
                 sc[t * DQ_LV + s] = gap >= 0 ? s4[i][j] * lp[gap] : 0.0f;
             }
         __syncthreads();
+        if (diag && odd) {
+            // A value that is no number or infinite: 0 x infinity would carry it into tokens before it (the scores above the
+            // diagonal are zeros), so every later token is left out. The same sums in the same order. (Leaving them out always
+            // made the three kernels 3.5 % slower over 162 shapes, this check 0 %.)
+#pragma unroll 1
+            for (int s = 0; s < DQ_T; s++) {
+                float v1[4];
+#pragma unroll
+                for (int j = 0; j < 4; j++) v1[j] = vt[(tx + 16 * j) * DQ_LV + s];
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const float p = sc[(ty + 16 * i) * DQ_LV + s];
+#pragma unroll
+                    for (int j = 0; j < 4; j++)
+                        if (s <= ty + 16 * i) o[i][j] = fmaf(p, v1[j], o[i][j]);
+                }
+            }
+            continue;
+        }
 #pragma unroll
         for (int sb = 0; sb < 4; sb++)
 #pragma unroll

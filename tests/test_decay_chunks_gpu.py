@@ -46,3 +46,39 @@ def test_tiles_of_tokens_against_the_recurrence(H, d, dv, lens, dtype, planes, c
             # 32-bit sums of up to n + d terms, rounded silu (2^-21) in every factor: far below 1e-5 of the terms' sum
             assert float(((out[t].view(H, dv).double() - want).abs() / (most + 1e-30)).max()) < 1e-5, (b, t)
         assert float(((state[int(slots[b])].double().transpose(1, 2) - S).abs() / (size + 1e-30)).max()) < 1e-5, b
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+@pytest.mark.parametrize("dtype,chunk", [("bfloat16", 64), ("bfloat16", 128), ("float32", 64), ("bfloat16", 48)])
+def test_what_is_not_finite_stays_out_of_earlier_tokens(dtype, chunk, bad):
+    """a value, key or query that is no number or infinite changes no earlier token, and a value no other column"""
+    from kindi_b200.kernels import lib as K
+    K.load()
+    H, d, dv, T = 2, 64, 72, 150
+    g = torch.Generator(device="cuda").manual_seed(chunk)
+    clean = torch.randn(T, 2 * H * d + H * dv, device="cuda", generator=g).to(getattr(torch, dtype))
+    decay = torch.tensor([1.0, 0.95], device="cuda")
+    q_start = torch.tensor([0, T], dtype=torch.int32, device="cuda")
+    state0 = torch.randn(1, H, dv, d, device="cuda", generator=g)
+
+    def go(x):
+        out = torch.full((T, H * dv), float("nan"), device="cuda")
+        K.decay_scan(x, 1, H, d, dv, decay, q_start, torch.zeros(1, dtype=torch.int32, device="cuda"), state0.clone(), out,
+                     chunk=chunk, max_rows=T)
+        return out.view(T, H, dv)
+    want = go(clean)
+    assert bool(want.isfinite().all())
+    for s in (1, 15, 16, 37, 63, 64, 79, 127, T - 1):
+        for kind, col in (("v", 2 * H * d + 5), ("v", 2 * H * d + dv + 70), ("k", H * d + 3), ("q", d + 1)):
+            x = clean.clone()
+            x[s, col] = bad
+            got = go(x)
+            h = {"v": (col - 2 * H * d) // dv, "k": (col - H * d) // d, "q": col // d}[kind]
+            assert torch.equal(got[:s], want[:s]), (kind, s)
+            assert torch.equal(got[:, 1 - h], want[:, 1 - h]), (kind, s)
+            if kind == "v":
+                e = (col - 2 * H * d) % dv
+                others = [c for c in range(dv) if c != e]
+                assert torch.equal(got[:, :, others], want[:, :, others]), s
+            if kind == "q":
+                assert torch.equal(got[s + 1:], want[s + 1:]), s
