@@ -650,6 +650,24 @@ def test_norm_of_rows_shared_by_warps(K, kind, T, E, planes, scaled):
         assert float(((y.double() - want).abs() / (want.abs() + 1e-2)).max()) < 2 ** -8
 
 
+@pytest.mark.parametrize("T,E,planes", [(64, 3076, 1), (67, 4096, 3), (64, 5120, 1), (65, 6144, 2), (160, 2052, 2), (163, 2560, 1),
+                                        (161, 3072, 5), (600, 4100, 0)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_layer_norm_of_wide_rows_adds_in_the_block_forms_order(K, T, E, planes, dtype):
+    """rows shared by several warps give the bits of the block per row (which steps that pick rows take), so that what a
+    router picks behind the norm does not depend on the step's rows"""
+    g = torch.Generator(device="cuda").manual_seed(T + E)
+    x0 = torch.randn(T, E, device="cuda", generator=g) + 0.5
+    d = torch.randn(planes, T, E, device="cuda", generator=g) if planes else None
+    w, b = (torch.randn(2, E, device="cuda", generator=g) + 1).to(dtype)
+    got = []
+    for rows in (None, torch.arange(T, dtype=torch.int32, device="cuda")):
+        x, y = x0.clone(), torch.empty(T, E, device="cuda", dtype=torch.bfloat16)
+        K.add_layernorm(x, d, w, b, 1e-5, y, rows, d is not None and rows is None, _status())
+        got.append(y)
+    assert torch.equal(got[0], got[1])
+
+
 def test_page_table_entries_from_pinned_memory(K):
     table = torch.full((3, 700), -1, dtype=torch.int32, device="cuda")
     want = table.clone()
