@@ -386,8 +386,7 @@ __global__ void __launch_bounds__(256) k_add_rmsnorm_warp(float* KB_STEP_DATA x,
 #define NORM_ROWS_MIN_T 160
 
 // (norm_rows.cu)
-bool kb_norm_rows_takes(const void* x, const void* delta, int n_delta, long long stride, const void* w, int wdtype, const void* y,
-                        int E);
+bool kb_norm_rows_takes(const void* x, const void* delta, int n_delta, long long stride, const void* y, int E);
 int kb_norm_rows(float* x, const float* delta, int n_delta, size_t stride, const void* w, const void* bias, int wdtype, float eps,
                  void* y, int T, int E, const void* ls, bool layer_norm, cudaStream_t st);
 
@@ -403,7 +402,7 @@ extern "C" int kb_add_rmsnorm(float* x, const float* delta, int n_delta, long lo
                      (delta_stride % 4 == 0);
     cudaError_t e = cudaSuccess;
     if (ydtype == KB_BF16 && rows == nullptr && n_out == T && T >= NORM_ROWS_MIN_T && (write_back || n_delta == 0) &&
-        kb_norm_rows_takes(x, delta, n_delta, delta_stride, w, wdtype, y, E))
+        kb_norm_rows_takes(x, delta, n_delta, delta_stride, y, E))
         return kb_norm_rows(x, delta, n_delta, (size_t)delta_stride, w, nullptr, wdtype, eps, y, T, E, ls, false, st);
     if (ydtype == KB_BF16 && vec && rows == nullptr && n_out == T && T >= 512 && (write_back || n_delta == 0) &&
         (((uintptr_t)y) % 8) == 0) {

@@ -19,7 +19,8 @@
 enum { NR_RMS, NR_LN_LANES, NR_LN_BLOCK };
 #define NR_BLOCK_WARPS 16               // of k_add_layernorm
 
-template <typename TW, int WPR, int NC, int PB, int KIND, int MINB>
+// G4: the gains lie on boundaries of four (their loads are then asked for early, before the sums)
+template <typename TW, int WPR, int NC, int PB, int KIND, int MINB, bool G4>
 __global__ void __launch_bounds__(256, MINB) k_norm_rows(float* KB_STEP_DATA x, const float* KB_STEP_DATA delta, int n_delta,
         size_t delta_stride, const TW* __restrict__ w, const TW* __restrict__ bias, float eps, bf16* __restrict__ y, int T, int E,
         const TW* __restrict__ ls) {
@@ -141,7 +142,10 @@ __global__ void __launch_bounds__(256, MINB) k_norm_rows(float* KB_STEP_DATA x, 
         const int i = i0 + STEP * c;
         if (i >= E) continue;
         float g[4], o[4] = {v[c].x, v[c].y, v[c].z, v[c].w};
-        if (sizeof(TW) == 2) {
+        if (!G4) {
+#pragma unroll
+            for (int k = 0; k < 4; k++) g[k] = kb_to_f<TW>(w[i + k]);
+        } else if (sizeof(TW) == 2) {
             const uint2 r = *(const uint2*)(w + i);
             const float2 a = __bfloat1622float2(*(const __nv_bfloat162*)&r.x), b = __bfloat1622float2(*(const __nv_bfloat162*)&r.y);
             g[0] = a.x; g[1] = a.y; g[2] = b.x; g[3] = b.y;
@@ -159,11 +163,11 @@ __global__ void __launch_bounds__(256, MINB) k_norm_rows(float* KB_STEP_DATA x, 
     }
 }
 
-template <typename TW, bool LN>
-static int norm_rows(float* x, const float* delta, int n_delta, size_t stride, const TW* w, const TW* bias, float eps, bf16* y, int T,
+template <typename TW, bool LN, bool G4>
+static int norm_rows_of(float* x, const float* delta, int n_delta, size_t stride, const TW* w, const TW* bias, float eps, bf16* y, int T,
                      int E, const TW* ls, cudaStream_t st) {
 #define NR_GO(WPR, NC, PB, MINB)                                                                                       \
-    return (int)kb_launch(k_norm_rows<TW, WPR, NC, PB, !LN ? NR_RMS : WPR * NC <= 16 ? NR_LN_LANES : NR_LN_BLOCK, MINB>, \
+    return (int)kb_launch(k_norm_rows<TW, WPR, NC, PB, !LN ? NR_RMS : WPR * NC <= 16 ? NR_LN_LANES : NR_LN_BLOCK, MINB, G4>, \
                           (T + 8 / WPR - 1) / (8 / WPR), 256, 0, st, x, delta, n_delta, stride, w, bias, eps, y, T, E, ls)
     if (n_delta <= 1) {
         if (E <= 1024) NR_GO(4, 2, 1, 6);
@@ -180,11 +184,17 @@ static int norm_rows(float* x, const float* delta, int n_delta, size_t stride, c
 #undef NR_GO
 }
 
-// whether k_norm_rows takes the operands (E up to 6144; x, planes and stride in 16-byte pieces, gains and y in 4 elements)
-bool kb_norm_rows_takes(const void* x, const void* delta, int n_delta, long long stride, const void* w, int wdtype, const void* y,
-                        int E) {
+template <typename TW, bool LN>
+static int norm_rows(float* x, const float* delta, int n_delta, size_t stride, const TW* w, const TW* bias, float eps, bf16* y, int T,
+                     int E, const TW* ls, cudaStream_t st) {
+    return ((uintptr_t)w & (sizeof(TW) * 4 - 1)) == 0 ? norm_rows_of<TW, LN, true>(x, delta, n_delta, stride, w, bias, eps, y, T, E, ls, st)
+                                                      : norm_rows_of<TW, LN, false>(x, delta, n_delta, stride, w, bias, eps, y, T, E, ls, st);
+}
+
+// whether k_norm_rows takes the operands (E up to 6144; x, planes and stride in 16-byte pieces, y in 4 elements)
+bool kb_norm_rows_takes(const void* x, const void* delta, int n_delta, long long stride, const void* y, int E) {
     return E % 4 == 0 && E <= 6144 && ((uintptr_t)x & 15) == 0 && (n_delta == 0 || (((uintptr_t)delta & 15) == 0 && stride % 4 == 0)) &&
-           ((uintptr_t)w & (wdtype == KB_F32 ? 15 : 7)) == 0 && ((uintptr_t)y & 7) == 0;
+           ((uintptr_t)y & 7) == 0;
 }
 
 int kb_norm_rows(float* x, const float* delta, int n_delta, size_t stride, const void* w, const void* bias, int wdtype, float eps,

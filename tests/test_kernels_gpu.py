@@ -625,7 +625,7 @@ def test_rotation_angles_of_a_step_are_the_kernels_own(K):
                                                (171, 4096, 2, False), (163, 4100, 1, False), (160, 6144, 9, True), (160, 6148, 1, False)])
 def test_norm_of_rows_shared_by_warps(K, kind, T, E, planes, scaled):
     """every split of a row over warps, at its widest and just above, with rows that do not fill the last block, gains that are
-    aligned and gains that are not (those keep the block per row)"""
+    aligned and gains that are not"""
     if kind == "layer" and scaled:
         scaled = False
     g = torch.Generator(device="cuda").manual_seed(T * 10000 + E)
@@ -666,6 +666,26 @@ def test_layer_norm_of_wide_rows_adds_in_the_block_forms_order(K, T, E, planes, 
         K.add_layernorm(x, d, w, b, 1e-5, y, rows, d is not None and rows is None, _status())
         got.append(y)
     assert torch.equal(got[0], got[1])
+
+
+@pytest.mark.parametrize("kind", ["rms", "layer"])
+@pytest.mark.parametrize("T,E", [(160, 1024), (200, 2048), (165, 2560), (512, 4096), (161, 5120), (1800, 1028)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_norm_gains_that_start_anywhere_give_the_same_bits(K, kind, T, E, dtype):
+    g = torch.Generator(device="cuda").manual_seed(T + E)
+    x0, d = torch.randn(T, E, device="cuda", generator=g), torch.randn(2, T, E, device="cuda", generator=g)
+    w, b = (torch.randn(2, E, device="cuda", generator=g) + 1).to(dtype)
+    got = []
+    for at in (0, 1, 2, 3):
+        store = torch.empty(E + 4, device="cuda", dtype=dtype)
+        store[at:at + E] = w
+        x, y = x0.clone(), torch.empty(T, E, device="cuda", dtype=torch.bfloat16)
+        if kind == "rms":
+            K.add_rmsnorm(x, d, store[at:at + E], 1e-5, y, None, True, _status())
+        else:
+            K.add_layernorm(x, d, store[at:at + E], b, 1e-5, y, None, True, _status())
+        got.append(y)
+    assert all(torch.equal(got[0], y) for y in got[1:])
 
 
 def test_page_table_entries_from_pinned_memory(K):
