@@ -381,8 +381,10 @@ __global__ void __launch_bounds__(256) k_add_rmsnorm_warp(float* KB_STEP_DATA x,
     }
 }
 
-// Rows of a step from which several warps share a row (norm_rows.cu, widths up to 6144). Below, a block per row is as fast:
-// 128 rows of 2560 with one plane 2.6 us against 3.6, 160 rows 4.2 against 3.7.
+// Rows of a step from which several warps share a row (norm_rows.cu, widths up to 6144): the first multiple of 32 above the
+// SMs. A block per row that has an SM to itself is as fast up to 2560 columns (128 rows of 2560: 2.8 us against 2.5 with one
+// plane, 2.8 against 3.2 with four); with two on an SM it is not (160 rows: 4.5 against 2.2, 4.6 against 2.9). Wider rows
+// would gain below the line too (128 rows of 4096: 3.3 against 2.3 us); a step that small keeps the block's order.
 #define NORM_ROWS_MIN_T 160
 
 // (norm_rows.cu)

@@ -87,8 +87,11 @@ __global__ void __launch_bounds__(LN_THREADS) k_add_layernorm(float* KB_STEP_DAT
 }
 
 // Rows of a bfloat16 step from which several warps share a row (norm_rows.cu, widths up to 6144); the true 32-bit path, whose
-// results must not depend on how many rows a step has, never uses it.
-#define LN_ROWS_MIN_T 64
+// results must not depend on how many rows a step has, never uses it. Widths of 2049 to 3072 have four warps a row there with
+// six pieces a thread: below 160 rows the block per row is as fast with one plane and faster with more (128 rows of 2560 with
+// four planes 3.6 us against 4.3; 160: 4.4 and 4.4; 320: 6.5 against 4.8). Others gain from 64 rows on (64 rows of 4096: 3.6
+// us against 3.1).
+#define LN_ROWS_MIN_T(E) ((E) > 2048 && (E) <= 3072 ? 160 : 64)
 
 // (norm_rows.cu)
 bool kb_norm_rows_takes(const void* x, const void* delta, int n_delta, long long stride, const void* y, int E);
@@ -104,7 +107,7 @@ extern "C" int kb_add_layernorm(float* x, const float* delta, int n_delta, long 
     const int vec = (E % 4 == 0) && (((uintptr_t)x) % 16 == 0) && (((uintptr_t)delta) % 16 == 0) &&
                     (delta_stride % 4 == 0);
     cudaError_t e = cudaSuccess;
-    if (ydtype == KB_BF16 && rows == nullptr && n_out == T && T >= LN_ROWS_MIN_T && (write_back || n_delta == 0) &&
+    if (ydtype == KB_BF16 && rows == nullptr && n_out == T && T >= LN_ROWS_MIN_T(E) && (write_back || n_delta == 0) &&
         kb_norm_rows_takes(x, delta, n_delta, delta_stride, y, E))
         return kb_norm_rows(x, delta, n_delta, (size_t)delta_stride, w, bias, wdtype, eps, y, T, E, nullptr, true, st);
 #define KB_LN(TY, TW)                                                                                              \

@@ -177,9 +177,9 @@ static int norm_rows_of(float* x, const float* delta, int n_delta, size_t stride
         NR_GO(8, 6, 1, 4);
     }
     if (E <= 1024) NR_GO(4, 2, 4, 4);
-    if (E <= 2048) NR_GO(4, 4, 2, 3);
+    if (E <= 2048) NR_GO(4, 4, 2, 4);
     if (E <= 3072) NR_GO(4, 6, 2, 2);
-    if (E <= 4096) NR_GO(8, 4, 2, 3);
+    if (E <= 4096) NR_GO(8, 4, 2, 4);
     NR_GO(8, 6, 2, 2);
 #undef NR_GO
 }
