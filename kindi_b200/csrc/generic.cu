@@ -1038,15 +1038,16 @@ __global__ void __launch_bounds__(128) k_attn_generic(const T* KB_STEP_DATA q, i
 }
 
 bool kb_attn_rows_takes(const void* q, int ldq, const void* out, int ldo, const void* pool, int hd, int vd);
-int kb_attn_rows(const float* q, int ldq, float* out, int ldo, const int* pos, const int* seq, const int* slot, int T, int nkv,
-                 int group, int hd, float scale, int window, int keep_first, const KbCacheView& cv, int* status,
+int kb_attn_rows(const float* q, int ldq, float* out, int ldo, const int* pos, const int* seq, const int* slot, int T, int n_seq,
+                 int nkv, int group, int hd, float scale, int window, int keep_first, const KbCacheView& cv, int* status,
                  const float* sink, const float* gate, int ldg, int chunk, float cap, int vd, cudaStream_t st);
 
 extern "C" int kb_attn_generic(const void* q, int dtype, int ldq, void* out, int ldo, const int* pos, const int* seq,
                                const int* slot, int T, int nh, int nkv, int hd, float scale, int window, void* pool,
                                const int* table, int table_stride, int n_pages, int* status, cudaStream_t st,
                                int keep_first, const float* sink, const void* gate, int ldg, int chunk, float cap, int vd,
-                               int one_plane) {
+                               int one_plane, int n_seq) {
+    // n_seq: an upper bound of the step's sequences (entries of slot)
     // vd (0: hd): elements of a value, and of a head of the output. one_plane: values are their keys' beginnings. sink (float [nh] or null): exp(sink[h]) joins the softmax denominator of head h. gate (rows of the queries'
     // type [T][ldg], laid out like the output, or null): out *= 1 / (1 + exp(-gate))
     if (T <= 0) return 0;
@@ -1057,8 +1058,8 @@ extern "C" int kb_attn_generic(const void* q, int dtype, int ldq, void* out, int
     KbCacheView cv{pool, table, table_stride, n_pages, nkv, hd, one_plane};
     // 32-bit heads of up to 128 elements: the same arithmetic over tiles that rows share (attn_rows.cu)
     if (dtype == KB_F32 && kb_attn_rows_takes(q, ldq, out, ldo, pool, hd, vd))
-        return kb_attn_rows((const float*)q, ldq, (float*)out, ldo, pos, seq, slot, T, nkv, nh / nkv, hd, scale, window,
-                            keep_first, cv, status, sink, (const float*)gate, ldg, chunk, cap, vd, st);
+        return kb_attn_rows((const float*)q, ldq, (float*)out, ldo, pos, seq, slot, T, n_seq, nkv, nh / nkv, hd, scale,
+                            window, keep_first, cv, status, sink, (const float*)gate, ldg, chunk, cap, vd, st);
     long long items = (long long)T * nh;
     int grid = (int)((items + 3) / 4);
     if (dtype == KB_F32)

@@ -62,7 +62,7 @@ _SIGS = {
     "kb_rope_table": [c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p],
     "kb_attn_generic": [c_void_p, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
                         c_int, c_float, c_int, c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p, c_int, c_void_p,
-                        c_void_p, c_int, c_int, c_float, c_int, c_int],
+                        c_void_p, c_int, c_int, c_float, c_int, c_int, c_int],
     "kb_gate_mul": [c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_longlong, c_int, c_void_p, c_int, c_int, c_int,
                     c_void_p],
     "kb_gated_rmsnorm": [c_void_p, c_int, c_void_p, c_int, c_float, c_void_p, c_int, c_int, c_longlong, c_int, c_void_p,
@@ -846,7 +846,7 @@ def attn_generic(q: torch.Tensor, out: torch.Tensor, pos, seq, slot, nh: int, nk
                                   nh, nkv, hd, float(scale), int(window), _p(pool), _p(table), table.stride(0),
                                   n_pages, _p(status), _stream(), int(keep_first), _p(sink), _p(gate),
                                   gate.stride(0) if gate is not None else 0, int(chunk), float(softcap), int(v_dim),
-                                  1 if pool.dim() >= 4 and pool.shape[-4] == 1 else 0), "attn_generic")
+                                  1 if pool.dim() >= 4 and pool.shape[-4] == 1 else 0, slot.numel()), "attn_generic")
 
 
 LATENT_DIMS = (64, 128, 192, 256, 320, 576)       # sizes of a cached latent that the tensor-core kernels take

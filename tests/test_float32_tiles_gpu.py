@@ -94,3 +94,59 @@ def test_an_unmapped_page_is_reported_only_where_a_row_sees_it(K):
         st = torch.zeros(1, dtype=torch.int32, device="cuda")
         K.attn_generic(q, out, dev([130, 131]), dev([0, 0]), dev([0]), 1, 1, 32, 0.2, window, pool, dev([row]), 4, st)
         assert (int(st.item()) == K.ST_BAD_PAGE) == bad
+
+
+@pytest.mark.parametrize("nh,nkv,hd", [(16, 16, 64), (8, 2, 128), (40, 2, 32)])
+@pytest.mark.parametrize("q_lens", [[1] * 20, [1] * 9 + [50] + [1] * 9, [2] * 11, [40] + [1] * 15, [300] * 5, [3, 1, 17, 1, 1, 2]])
+def test_tiles_of_many_sequences(K, nh, nkv, hd, q_lens):
+    """single tokens, few tokens each, a prompt before, between and behind single tokens; also with the rows in no order"""
+    rng = random.Random(len(q_lens) + nh)
+    kv_lens = [n + rng.choice([0, 5, 64, 100]) for n in q_lens]
+    n_pages = sum(-(-n // 64) for n in kv_lens)
+    order = list(range(n_pages))
+    rng.shuffle(order)
+    g = torch.Generator(device="cuda").manual_seed(nh)
+    pool = torch.randn(n_pages, 2, nkv, 64, hd, device="cuda", generator=g)
+    table = torch.full((len(q_lens), 8), -1, dtype=torch.int32)
+    rows = []
+    for b, (ql, kl) in enumerate(zip(q_lens, kv_lens)):
+        for i in range(-(-kl // 64)):
+            table[b, i] = order.pop()
+        rows += [(p, b) for p in range(kl - ql, kl)]
+    dev = lambda x: torch.tensor(x, dtype=torch.int32).cuda()      # noqa: E731
+    for mixed in (False, True):
+        if mixed:
+            rng.shuffle(rows)
+        T = len(rows)
+        q = torch.randn(T, nh * hd, device="cuda", generator=g)
+        st = torch.zeros(1, dtype=torch.int32, device="cuda")
+        outs = [torch.full((T, nh * hd), 7.0, device="cuda"), torch.full((T, nh * hd + 1), 7.0, device="cuda")[:, :nh * hd]]
+        for out in outs:                                            # (rows of an odd stride run the general kernel)
+            K.attn_generic(q, out, dev([p for p, _ in rows]), dev([b for _, b in rows]), dev(list(range(len(q_lens)))), nh, nkv,
+                           hd, 0.2, 0, pool, table.cuda(), n_pages, st)
+        assert torch.equal(outs[0], outs[1]) and int(st.item()) == 0
+
+
+@pytest.mark.parametrize("nh,nkv,hd", [(16, 16, 64), (8, 2, 128)])
+def test_single_tokens_of_many_sequences_run_side_by_side(K, nh, nkv, hd):
+    """the tiled form has no sequence wait for another one's chain of positions: it is no slower than the general kernel
+    (a tenth of its time when the sequences run side by side)"""
+    B, n = 16, 1000
+    pool = torch.randn(B * 16, 2, nkv, 64, hd, device="cuda")
+    table = torch.arange(B * 16, dtype=torch.int32, device="cuda").view(B, 16)
+    dev = lambda x: torch.tensor(x, dtype=torch.int32).cuda()      # noqa: E731
+    pos, seq, q = dev([n - 1] * B), dev(list(range(B))), torch.randn(B, nh * hd, device="cuda")
+    st = torch.zeros(1, dtype=torch.int32, device="cuda")
+    times = []
+    for out in (torch.empty(B, nh * hd, device="cuda"), torch.empty(B, nh * hd + 1, device="cuda")[:, :nh * hd]):
+        best = float("inf")
+        for _ in range(6):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            for _ in range(5):
+                K.attn_generic(q, out, pos, seq, seq, nh, nkv, hd, 0.2, 0, pool, table, B * 16, st)
+            b.record()
+            torch.cuda.synchronize()
+            best = min(best, a.elapsed_time(b))
+        times.append(best)
+    assert times[0] < times[1]
