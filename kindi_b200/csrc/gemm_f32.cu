@@ -130,15 +130,24 @@ static int launch_f32(const float* A, const float* W, float* C, int M, int N, in
     KB_LAUNCH_RET();
 }
 
-// The tiles, and what a unit of 1024 K elements takes on an SM, in microseconds: alone, and beside enough others (measured
-// at N = 32768; large products reach 44 TFLOP/s). Few units want small tiles: 514 x 1024 outputs over K = 1024 take 80 us in
-// tiles of 64 x 128 and 61 to 69 us in tiles of 32 x 32 or 16 x 64; four rows of 5632 columns 70 against 14 us.
-struct F32Choice { int bm, bn; float alone, each; };
-static const F32Choice kF32Tiles[] = {{64, 128, 70.f, 54.f}, {64, 64, 37.f, 28.f}, {32, 64, 24.f, 15.3f}, {32, 32, 17.f, 9.4f},
-                                      {16, 64, 18.f, 10.6f}, {16, 32, 13.4f, 9.7f}, {8, 64, 14.f, 10.5f}, {4, 64, 11.8f, 8.5f}};
+// The tiles, and what a product over 1024 K elements takes on them, in microseconds, by the rounds of units (ceil(units / SMs));
+// measured at 1 to 2048 rows of 8 to 32768 columns over K = 256, 1024 and 4096. Within the first round a lone unit on its SM
+// takes `few` while up to six tenths of the SMs have one, `full` beyond: the thin tiles fetch the most for a product and share
+// the way from the L2. The tile that this picks is 1.0 % slower than the best of the eight on average over those 440 products
+// (costs of a lone and of an added unit, with a charge from 90 units on: 3.8 %). 514 x 1024 outputs over K = 1024 take 73 us in
+// tiles of 64 x 128, 42 in 64 x 64 (144 units, chosen), 44 in 32 x 64, 59 in 32 x 32; 514 x 256 71, 39, 24 and 19 (chosen).
+struct F32Choice { int bm, bn; float few, full, two, three, four, more; };
+static const F32Choice kF32Tiles[] = {{64, 128, 72.f, 72.f, 126.f, 162.f, 226.f, 38.f}, {64, 64, 40.f, 41.f, 70.f, 106.f, 115.f, 26.f},
+                                      {32, 64, 24.f, 26.f, 43.f, 58.f, 81.f, 12.f}, {32, 32, 16.6f, 18.f, 26.f, 37.5f, 57.f, 8.4f},
+                                      {16, 64, 17.7f, 20.5f, 27.7f, 37.6f, 55.f, 8.4f}, {16, 32, 13.f, 16.3f, 30.f, 41.f, 48.5f, 11.f},
+                                      {8, 64, 13.9f, 20.f, 30.f, 33.f, 52.f, 9.5f}, {4, 64, 11.4f, 15.f, 24.f, 26.f, 34.6f, 9.f}};
 
-// the tile of the least estimated time: whole rounds of units while they are few; and units beyond the first on an SM share
-// it unevenly (six tenths of a lone unit's time, measured)
+static float f32_cost(const F32Choice& t, int M, int N, int sms) {
+    const long long units = (long long)((M + t.bm - 1) / t.bm) * ((N + t.bn - 1) / t.bn), rounds = (units + sms - 1) / sms;
+    if (rounds <= 1) return 10 * units <= 6 * sms ? t.few : t.full;
+    return rounds == 2 ? t.two : rounds == 3 ? t.three : t.four + (float)(rounds - 4) * t.more;
+}
+// the tile of the least estimated time
 static int f32_tile(int M, int N) {
     static int sms = 0;
     if (!sms) {
@@ -146,14 +155,11 @@ static int f32_tile(int M, int N) {
         cudaGetDevice(&dev);
         if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
     }
-    int best = 0;
+    int best = -1;
     float best_cost = 0.0f;
     for (int i = 0; i < (int)(sizeof(kF32Tiles) / sizeof(kF32Tiles[0])); i++) {
-        const F32Choice& t = kF32Tiles[i];
-        const long long units = (long long)((M + t.bm - 1) / t.bm) * ((N + t.bn - 1) / t.bn);
-        const float rounds = units <= 4 * sms ? (float)((units + sms - 1) / sms) : (float)units / (float)sms;
-        const float cost = (rounds * t.each > t.alone ? rounds * t.each : t.alone) + (units > 90 ? 0.6f * t.alone : 0.0f);
-        if (i == 0 || cost < best_cost) {
+        const float cost = f32_cost(kF32Tiles[i], M, N, sms);
+        if (best < 0 || cost < best_cost) {
             best = i;
             best_cost = cost;
         }

@@ -150,3 +150,21 @@ def test_single_tokens_of_many_sequences_run_side_by_side(K, nh, nkv, hd):
             best = min(best, a.elapsed_time(b))
         times.append(best)
     assert times[0] < times[1]
+
+
+@pytest.mark.parametrize("M,N,K_", [(2048, 64, 4096), (514, 256, 4096), (64, 1536, 4096), (257, 256, 4096), (514, 1024, 1024)])
+def test_the_chosen_tile_is_near_the_best(K, M, N, K_):
+    """products of about as many units as there are SMs, on both sides of the lines between tiles: the choice is within a fifth
+    of the best of the eight (timed; 1.00 to 1.03 when written down)"""
+    a, w, out = torch.randn(M, K_, device="cuda"), torch.randn(N, K_, device="cuda"), torch.empty(M, N, device="cuda")
+    best = [float("inf")] * 9
+    for _ in range(5):
+        for tile in range(-1, 8):
+            x, y = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            x.record()
+            for _ in range(10):
+                K.gemm_f32(a, w, out, tile)
+            y.record()
+            torch.cuda.synchronize()
+            best[tile + 1] = min(best[tile + 1], x.elapsed_time(y))
+    assert best[0] < 1.2 * min(best[1:]), best
