@@ -147,7 +147,7 @@ static float f32_cost(const F32Choice& t, int M, int N, int sms) {
     if (rounds <= 1) return 10 * units <= 6 * sms ? t.few : t.full;
     return rounds == 2 ? t.two : rounds == 3 ? t.three : t.four + (float)(rounds - 4) * t.more;
 }
-// the tile of the least estimated time
+// the tile of the least estimated time among those whose grid is not too tall, or -1
 static int f32_tile(int M, int N) {
     static int sms = 0;
     if (!sms) {
@@ -158,6 +158,7 @@ static int f32_tile(int M, int N) {
     int best = -1;
     float best_cost = 0.0f;
     for (int i = 0; i < (int)(sizeof(kF32Tiles) / sizeof(kF32Tiles[0])); i++) {
+        if ((M + kF32Tiles[i].bm - 1) / kF32Tiles[i].bm > 65535) continue;
         const float cost = f32_cost(kF32Tiles[i], M, N, sms);
         if (best < 0 || cost < best_cost) {
             best = i;

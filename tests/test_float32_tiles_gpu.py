@@ -168,3 +168,15 @@ def test_the_chosen_tile_is_near_the_best(K, M, N, K_):
             torch.cuda.synchronize()
             best[tile + 1] = min(best[tile + 1], x.elapsed_time(y))
     assert best[0] < 1.2 * min(best[1:]), best
+
+
+def test_a_product_of_very_many_rows(K):
+    """rows whose tiles of 32 would make too tall a grid (65535 blocks)"""
+    M, N, K_ = 2_100_000, 4, 4
+    a, w, out = torch.randn(M, K_, device="cuda"), torch.randn(N, K_, device="cuda"), torch.empty(M, N, device="cuda")
+    K.gemm_simt(a, w, out)
+    odd = torch.empty(M, K_ + 1, device="cuda")[:, :K_]
+    odd.copy_(a)
+    want = torch.empty(M, N, device="cuda")
+    K.gemm_simt(odd, w, want)
+    assert torch.equal(out, want)
