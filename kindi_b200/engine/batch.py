@@ -98,10 +98,13 @@ def pack(entries: Sequence[StepEntry], length_before: Sequence[int], pad_rows_to
     kv_len = []
     for b, (e, n) in enumerate(zip(entries, q_len)):
         a = q_start[b]
-        try:
-            tok[a:a + n] = array("i", e.tokens)      # (a third faster than numpy's own walk over a tuple)
-        except TypeError:
-            tok[a:a + n] = e.tokens                  # (numbers that are no Python or numpy integers)
+        toks = e.tokens
+        if type(toks) is tuple or type(toks) is list:        # (others hold bytes or wrap around: numpy's rules)
+            try:
+                toks = array("i", toks)                      # (a third faster than numpy's own walk over a tuple)
+            except TypeError:
+                pass                                         # (numbers that are no Python or numpy integers)
+        tok[a:a + n] = toks
         pos[a:a + n] = np.arange(length_before[b], length_before[b] + n, dtype=np.int32)
         seq[a:a + n] = b
         kv_len.append(length_before[b] + n)

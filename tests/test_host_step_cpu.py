@@ -42,3 +42,18 @@ def test_token_ids_in_any_form(form):
     ps = pack([StepEntry(0, form(toks), (3,)), StepEntry(1, form((5, 6)), ())], [0, 2])
     a, n = ps.off["tok"]
     assert ps.meta[a:a + n].tolist() == [3, 0, 70000, 9, 5, 6]
+
+
+@pytest.mark.parametrize("toks,want", [
+    (bytearray([1, 2, 3, 4]), [1, 2, 3, 4]), (memoryview(bytes([7, 0, 9])), [7, 0, 9]), (np.array([5, 2 ** 31 + 3, 1]), [5, 3 - 2 ** 31, 1]),
+    (np.array([[4, 5]], dtype=np.uint8)[0], [4, 5]), (range(3, 6), [3, 4, 5])])
+def test_token_ids_that_are_no_tuple_keep_numpys_rules(toks, want):
+    """bytes are numbers, and an id beyond 32 bits in an array wraps around to one that the device reports"""
+    ps = pack([StepEntry(0, toks, ()), StepEntry(1, (8, 9), ())], [0, 0])
+    a, n = ps.off["tok"]
+    assert ps.meta[a:a + n].tolist() == want + [8, 9]
+
+
+def test_ids_beyond_32_bits_in_a_tuple_are_refused():
+    with pytest.raises(OverflowError):
+        pack([StepEntry(0, (1, 2 ** 31), ())], [0])
