@@ -390,7 +390,6 @@ static int launch_decay(const TIN* in, const DqRows& a, int B, const float* deca
     const int eb = (a.dv + DQ_E - 1) / DQ_E, per = (a.C + DQ_T - 1) / DQ_T;
     const size_t smem_add = (size_t)(DQ_T * (D + DQ_E) + a.C + 1) * sizeof(float);
     const size_t smem = (size_t)(2 * DQ_T * (D + 4) + 2 * DQ_T * DQ_LV + per * DQ_T + 1) * sizeof(float);
-    if (smem > 227 * 1024 || smem_add > 227 * 1024) return (int)cudaErrorInvalidValue;
     cudaError_t e;
     static char once_tag;
     if (kb_first_use(&once_tag)) {
@@ -411,12 +410,19 @@ static int launch_decay(const TIN* in, const DqRows& a, int B, const float* deca
     KB_LAUNCH_RET();
 }
 
+// whether the tiles take chunks of C tokens, at most nc_max of them a sequence: grids and shared memory (the powers of the decay)
+bool kb_decay_tiles_takes(int d, int C, int nc_max) {
+    const long long per = (C + DQ_T - 1) / DQ_T, D = d <= 64 ? 64 : 128;
+    return d <= 128 && nc_max * per <= 65535 && (DQ_T * (D + DQ_E) + C + 1) * 4 <= 227 * 1024 &&
+           (2 * DQ_T * (D + 4) + 2 * DQ_T * DQ_LV + per * DQ_T + 1) * 4 <= 227 * 1024;
+}
+
 // P: float [B][H][nc_max][dv][d]
 int kb_decay_tiles(const void* in, int in_dtype, int n_planes, size_t plane_stride, int ld_in, int B, int H, int d, int dv,
                    const float* decay, const int* q_start, const int* slot, float* state, float* P, float* out, int ldo, int C,
                    int nc_max, cudaStream_t st) {
     DqRows a{n_planes, plane_stride, ld_in, H, d, dv, C, nc_max, false, false};
-    if ((long long)nc_max * ((C + DQ_T - 1) / DQ_T) > 65535) return (int)cudaErrorInvalidValue;
+    if (!kb_decay_tiles_takes(d, C, nc_max)) return (int)cudaErrorInvalidValue;
     if (in_dtype == KB_BF16 && n_planes == 1 && ld_in % 8 == 0 && ((uintptr_t)in & 15) == 0 && d % 8 == 0) {
         a.vec_k = true;
         a.vec_v = dv % 8 == 0;

@@ -791,20 +791,22 @@ __global__ void __launch_bounds__(256) k_decay_prefix(int H, int d, int dv, cons
 }
 
 // (decay_chunk.cu)
+bool kb_decay_tiles_takes(int d, int C, int nc_max);
 int kb_decay_tiles(const void* in, int in_dtype, int n_planes, size_t plane_stride, int ld_in, int B, int H, int d, int dv,
                    const float* decay, const int* q_start, const int* slot, float* state, float* P, float* out, int ldo, int C,
                    int nc_max, cudaStream_t st);
 
 // chunked form: C = tokens of a chunk, nc_max = the most chunks a sequence of this step can have (the longest
 // sequence's; an upper bound is fine), P (float [B][H][nc_max][dv][d]) and S0 (float [B][H][dv][d]) scratch. Key sizes up to
-// 128 run as matrix products over tiles of tokens (decay_chunk.cu), larger ones with a warp per column of the state
+// 128 run as matrix products over tiles of tokens (decay_chunk.cu); larger ones, and chunks too long or too many for the tiles'
+// shared memory and grids (from 32,449 tokens on, or more than 65535 tiles a sequence), with a warp per column of the state
 extern "C" int kb_decay_chunked(const void* in, int in_dtype, int n_planes, long long plane_stride, int ld_in, int B,
                                 int H, int d, int dv, const float* decay, const int* q_start, const int* slot,
                                 float* state, float* P, float* S0, float* out, int ldo, int C, int nc_max,
                                 cudaStream_t st) {
     if (B <= 0 || H <= 0 || nc_max <= 0) return 0;
     if (d > 32 * DS_MAX_DPL || d <= 0 || dv <= 0 || C <= 0 || nc_max > 65535) return (int)cudaErrorInvalidValue;
-    if (d <= 128)
+    if (kb_decay_tiles_takes(d, C, nc_max))
         return kb_decay_tiles(in, in_dtype, n_planes, (size_t)plane_stride, ld_in, B, H, d, dv, decay, q_start, slot, state, P, out,
                               ldo, C, nc_max, st);
     dim3 grid(B * H, (dv + DC_COLS - 1) / DC_COLS, nc_max);

@@ -82,3 +82,25 @@ def test_what_is_not_finite_stays_out_of_earlier_tokens(dtype, chunk, bad):
                 assert torch.equal(got[:, :, others], want[:, :, others]), s
             if kind == "q":
                 assert torch.equal(got[s + 1:], want[s + 1:]), s
+
+
+@pytest.mark.parametrize("d,chunk,max_rows", [(8, 41000, 300), (128, 32448, 300), (128, 32449, 300), (72, 45000, 100000), (8, 65, 33000 * 65),
+                                              (8, 128, 32767 * 128)])
+def test_chunks_of_any_length_and_number(d, chunk, max_rows):
+    """chunks whose powers of the decay do not fit the tiles' shared memory, and more tiles than their grid takes"""
+    from kindi_b200.kernels import lib as K
+    K.load()
+    H, dv, lens = 1, 8, [130, 1]
+    g = torch.Generator(device="cuda").manual_seed(d)
+    x = torch.randn(sum(lens), 2 * H * d + H * dv, device="cuda", generator=g).to(torch.bfloat16)
+    decay, slots = torch.tensor([0.97], device="cuda"), torch.tensor([1, 0], dtype=torch.int32, device="cuda")
+    q_start = torch.tensor([0, 130, 131], dtype=torch.int32, device="cuda")
+    state0 = torch.randn(2, H, dv, d, device="cuda", generator=g)
+    got = []
+    for more in (dict(), dict(chunk=chunk, max_rows=max_rows)):
+        state, out = state0.clone(), torch.full((sum(lens), H * dv), float("nan"), device="cuda")
+        K.decay_scan(x, 2, H, d, dv, decay, q_start, slots, state, out, **more)
+        got.append((out, state))
+    for a, b in zip(*got):
+        # (the token-by-token form, whose sums are taken in another order)
+        assert float((a - b).abs().max() / a.abs().max()) < 1e-5
