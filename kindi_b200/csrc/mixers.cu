@@ -797,9 +797,12 @@ int kb_decay_tiles(const void* in, int in_dtype, int n_planes, size_t plane_stri
                    int nc_max, cudaStream_t st);
 
 // chunked form: C = tokens of a chunk, nc_max = the most chunks a sequence of this step can have (the longest
-// sequence's; an upper bound is fine), P (float [B][H][nc_max][dv][d]) and S0 (float [B][H][dv][d]) scratch. Key sizes up to
+// sequence's; an upper bound is fine), P (float [B][H][nc_max][dv][d]) and S0 (float [B][H][dv][d], see kb_decay_scratch) scratch. Key sizes up to
 // 128 run as matrix products over tiles of tokens (decay_chunk.cu); larger ones, and chunks too long or too many for the tiles'
 // shared memory and grids (from 32,449 tokens on, or more than 65535 tiles a sequence), with a warp per column of the state
+// states of scratch that kb_decay_chunked needs per (sequence, head): nc_max, and one more where the form copies the state first
+extern "C" int kb_decay_scratch(int d, int C, int nc_max) { return nc_max + (kb_decay_tiles_takes(d, C, nc_max) ? 0 : 1); }
+
 extern "C" int kb_decay_chunked(const void* in, int in_dtype, int n_planes, long long plane_stride, int ld_in, int B,
                                 int H, int d, int dv, const float* decay, const int* q_start, const int* slot,
                                 float* state, float* P, float* S0, float* out, int ldo, int C, int nc_max,

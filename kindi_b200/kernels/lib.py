@@ -83,6 +83,7 @@ _SIGS = {
     "kb_head_gemm": [c_void_p, c_int, c_int, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int,
                      c_int, c_void_p, c_int, c_int, c_longlong, c_int, c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_int,
                      c_int, c_int, c_void_p, c_float, c_int, c_void_p],
+    "kb_decay_scratch": [c_int, c_int, c_int],
     "kb_decay_chunked": [c_void_p, c_int, c_int, c_longlong, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
                          c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p],
     "kb_decay_scan": [c_void_p, c_int, c_int, c_longlong, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
@@ -618,9 +619,10 @@ def decay_scan(a: torch.Tensor, B: int, H: int, d: int, dv: int, decay: torch.Te
         raise KernelError("kindi_b200: linear attention supports key sizes up to 256, found %d" % d)
     if chunk > 0:
         nc = max(1, -(-int(max_rows) // chunk))
-        scratch = torch.empty((B * H * (nc + 1), dv, d), dtype=torch.float32, device=out.device)
+        states = load().kb_decay_scratch(d, chunk, nc)
+        scratch = torch.empty((B * H * states, dv, d), dtype=torch.float32, device=out.device)
         _check(load().kb_decay_chunked(_p(a), dt(a), n_planes, pstride, ld, B, H, d, dv, _p(decay), _p(q_start),
-                                       _p(slot), _p(state), _p(scratch), _p(scratch[B * H * nc:]), _p(out),
+                                       _p(slot), _p(state), _p(scratch), _p(scratch[B * H * nc:] if states > nc else None), _p(out),
                                        out.stride(0), chunk, nc, _stream()), "decay_chunked")
         add_launches(2)
         return

@@ -104,3 +104,20 @@ def test_chunks_of_any_length_and_number(d, chunk, max_rows):
     for a, b in zip(*got):
         # (the token-by-token form, whose sums are taken in another order)
         assert float((a - b).abs().max() / a.abs().max()) < 1e-5
+
+
+@pytest.mark.parametrize("d,copies", [(128, 0), (129, 1)])
+def test_scratch_is_what_the_form_reads(d, copies):
+    from kindi_b200.kernels import lib as K
+    K.load()
+    B, H, dv, n, chunk = 4, 8, 256, 60, 64
+    x = torch.randn(B * n, 2 * H * d + H * dv, device="cuda").to(torch.bfloat16)
+    q_start = torch.arange(B + 1, dtype=torch.int32, device="cuda") * n
+    slot = torch.arange(B, dtype=torch.int32, device="cuda")
+    state, out = torch.zeros(B, H, dv, d, device="cuda"), torch.empty(B * n, H * dv, device="cuda")
+    decay = torch.full((H,), 0.9, device="cuda")
+    torch.cuda.reset_peak_memory_stats()
+    before = torch.cuda.memory_allocated()
+    K.decay_scan(x, B, H, d, dv, decay, q_start, slot, state, out, chunk=chunk, max_rows=n)
+    used = torch.cuda.max_memory_allocated() - before
+    assert state.nbytes * (1 + copies) <= used < state.nbytes * (1.5 + copies)
