@@ -11,7 +11,7 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("H,d,dv,lens,dtype,planes", [
     (2, 128, 128, [63, 64, 65, 1, 200], "bfloat16", 1), (2, 64, 200, [129, 255, 257], "bfloat16", 1),
     (3, 72, 40, [130, 0, 191], "bfloat16", 1), (2, 36, 70, [70, 128], "bfloat16", 1), (2, 128, 64, [300], "float32", 2),
-    (2, 8, 8, [193], "bfloat16", 1)])
+    (2, 8, 8, [193], "bfloat16", 1), (2, 72, 136, [140, 66], "float32", 1), (3, 40, 20, [129], "float32", 3)])
 def test_tiles_of_tokens_against_the_recurrence(H, d, dv, lens, dtype, planes, chunk):
     from kindi_b200.kernels import lib as K
     K.load()
