@@ -16,6 +16,7 @@ were given back are handed out again first. The reference's counterpart is one s
 from __future__ import annotations
 
 from dataclasses import dataclass
+import sys
 from typing import Dict, List, Optional, Sequence, Tuple
 
 import numpy as np
@@ -41,6 +42,9 @@ def split_needs(need, entry: int = -1):
             raise TypeError("cache entry %d asks for %r; a part's cache_need must be KVNeed, StateNeed, None or a "
                             "tuple of those" % (entry, n))
     return kv, states
+
+
+_left: List[torch.Tensor] = []          # staging memory of caches that went while something was being recorded
 
 
 @dataclass
@@ -172,13 +176,25 @@ class SequenceCache:
         # scatter issued one by one hold the host up for tens of microseconds before the step's first kernel
         stage = self._stage(sum(len(last) for _, last in todo))
         a = 0
-        for g, last in todo:
-            n = len(last)
-            self._stage_np[a:a + n, 0] = list(last)
-            self._stage_np[a:a + n, 1] = list(last.values())
-            K.table_set(g.table, stage[a:a + n], n)
-            a += n
-        self._stage_free.record()
+        try:
+            for g, last in todo:
+                n = len(last)
+                self._stage_np[a:a + n, 0] = list(last)
+                self._stage_np[a:a + n, 1] = list(last.values())
+                K.table_set(g.table, stage[a:a + n], n)
+                a += n
+        finally:
+            self._stage_free.record()                        # (also behind the launches before one that failed)
+
+    def __del__(self):
+        # the kernels read the staging memory in place; the allocator, which knows of copies only, would hand it on at once
+        free = getattr(self, "_stage_free", None)
+        if free is None or sys.is_finalizing():
+            return
+        if torch.cuda.is_available() and torch.cuda.is_current_stream_capturing():
+            _left.append(self._stage_buf)                    # (a wait would end the recording: the few kilobytes stay)
+        else:
+            free.synchronize()
 
     def _stage(self, n: int) -> torch.Tensor:
         """pinned int32 staging memory of at least n pairs, free to be written (the copy out of it that was issued

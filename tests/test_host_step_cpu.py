@@ -3,8 +3,13 @@ none, and token ids in any numeric form are packed alike."""
 import numpy as np
 import pytest
 
+import torch
+
 from kindi_b200.cache.pages import CacheFull, FreeList, PageMap
+from kindi_b200.cache.sequence_cache import SequenceCache
 from kindi_b200.engine.batch import StepEntry, pack
+from kindi_b200.kernels import lib as K
+from kindi_b200.parts.base import KVNeed
 
 
 def test_many_ids_at_a_time_are_the_ones_taken_one_by_one():
@@ -57,3 +62,39 @@ def test_token_ids_that_are_no_tuple_keep_numpys_rules(toks, want):
 def test_ids_beyond_32_bits_in_a_tuple_are_refused():
     with pytest.raises(OverflowError):
         pack([StepEntry(0, (1, 2 ** 31), ())], [0])
+
+
+class _Event:
+    """stands in for the event behind the kernels that read the staging memory"""
+
+    def __init__(self):
+        self.recorded = self.waited = 0
+
+    def record(self):
+        self.recorded += 1
+
+    def synchronize(self):
+        self.waited += 1
+
+
+def test_staging_memory_is_kept_until_the_kernels_have_read_it():
+    cache = SequenceCache([KVNeed(1, 8, None)], max_tokens=128, n_slots=1, dtype=torch.float32, device="cpu")
+    event = cache._stage_free = _Event()
+    del cache
+    assert event.waited == 1
+
+
+def test_a_failed_launch_leaves_the_launches_before_it_waited_for(monkeypatch):
+    cache = SequenceCache([KVNeed(1, 8, None), KVNeed(2, 8, None)], max_tokens=128, n_slots=1, dtype=torch.float32, device="cpu")
+    stage, event, calls = torch.zeros(8, 2, dtype=torch.int32), _Event(), []
+
+    def table_set(table, entries, n):
+        calls.append(n)
+        if len(calls) == 2:
+            raise K.KernelError("no")
+    monkeypatch.setattr(K, "table_set", table_set)
+    cache.device, cache._stage, cache._stage_np, cache._stage_free = torch.device("cuda"), lambda n: stage, stage.numpy(), event
+    cache.reserve(cache.alloc_slot(), 100)
+    with pytest.raises(K.KernelError):
+        cache.flush()
+    assert calls == [2, 2] and event.recorded == 1
