@@ -15,8 +15,8 @@ were given back are handed out again first. The reference's counterpart is one s
 """
 from __future__ import annotations
 
-from dataclasses import dataclass
 import sys
+from dataclasses import dataclass
 from typing import Dict, List, Optional, Sequence, Tuple
 
 import numpy as np
@@ -58,6 +58,8 @@ class KVGroup:
 
 
 class SequenceCache:
+    STAGED_PLACES = 2 ** 31 - 1
+
     def __init__(self, needs: Sequence, *, max_tokens: int, n_slots: int, dtype: torch.dtype, device,
                  max_step_tokens: Optional[int] = None):
         """``needs[i]`` is the KVNeed / StateNeed / None of cache entry i. ``max_tokens`` is the most tokens all
@@ -167,10 +169,12 @@ class SequenceCache:
                 todo.append((g, {s * self.n_pages + b: pg for s, b, pg in dirty}))
         if not todo:
             return
-        if self.device.type != "cuda":
+        # (the staged places are 32-bit: a larger table takes the general way)
+        if self.device.type != "cuda" or self.n_slots * self.n_pages > self.STAGED_PLACES:
             for g, last in todo:
-                idx = torch.tensor(list(last), dtype=torch.int64)
-                g.table.view(-1).index_copy_(0, idx, torch.tensor(list(last.values()), dtype=torch.int32))
+                idx = torch.tensor(list(last), dtype=torch.int64, device=g.table.device)
+                pages = torch.tensor(list(last.values()), dtype=torch.int32, device=g.table.device)
+                g.table.view(-1).index_copy_(0, idx, pages)
             return
         # one launch a group that reads the places and the pages from pinned memory: a copy to the device, a conversion and a
         # scatter issued one by one hold the host up for tens of microseconds before the step's first kernel

@@ -98,3 +98,18 @@ def test_a_failed_launch_leaves_the_launches_before_it_waited_for(monkeypatch):
     with pytest.raises(K.KernelError):
         cache.flush()
     assert calls == [2, 2] and event.recorded == 1
+
+
+def test_a_table_of_more_places_than_32_bits_is_written_the_general_way(monkeypatch):
+    cache = SequenceCache([KVNeed(1, 8, None)], max_tokens=256, n_slots=2, dtype=torch.float32, device="cpu")
+    cache.device = torch.device("cuda")                      # (the table stays where it is)
+    monkeypatch.setattr(K, "table_set", lambda *a: pytest.fail("staged"))
+    monkeypatch.setattr(SequenceCache, "STAGED_PLACES", 7, raising=False)
+    monkeypatch.setattr(SequenceCache, "_stage", lambda self, n: pytest.fail("staged"))
+    slots = [cache.alloc_slot() for _ in range(2)]
+    for s in slots:
+        cache.reserve(s, 100)
+    cache.flush()
+    table = cache.groups[0].table
+    for s in slots:
+        assert table[s].tolist() == [cache.groups[0].pages.rows[s].get(b, -1) for b in range(4)]
