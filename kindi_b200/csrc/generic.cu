@@ -38,31 +38,40 @@ __global__ void k_embed(const TW* __restrict__ table, const int* __restrict__ to
     }
 }
 
-// The same row eight elements a thread (16 or 32 bytes in, 32 out, the same product): widths that are multiples of 8 with
-// aligned tables. An element a thread and pass made a row's loads wait for one another: eight rows of 2560 7.3 -> 2 us,
-// 2048 rows 12.1 -> 8.7 us, 8171 of 5120 84 -> 66 us (3.8 TB/s).
+// The same row eight elements a thread, in two pieces of four from the halves of 2048 columns (8 or 16 bytes in, 16 out, the same
+// product): widths that are multiples of 8 with aligned tables. An element a thread and pass made a row's loads wait for one another.
+// With the table in memory eight rows of 2560 take 6.3 -> 1.9 us, 2048 rows 15.5 -> 7.8, 8171 of 5120 89 -> 45; with it in the
+// L2 1024 rows of 2560 3.7 -> 3.0 (eight neighbouring elements a thread, whose stores fill every second 16 bytes: 4.3).
 template <typename TW>
 __global__ void __launch_bounds__(256) k_embed8(const TW* __restrict__ table, const int* __restrict__ tok, float* __restrict__ x,
                                                 int E, int vocab, float scale, int* status) {
     kb_pdl_launch();
     kb_pdl_wait();
-    const int t = blockIdx.x, c = (blockIdx.y * 256 + threadIdx.x) * 8;
-    if (c >= E) return;
+    const int t = blockIdx.x, base = blockIdx.y * 2048, half = min(2048, E - base) / 2, c0 = base + threadIdx.x * 4;
+    if (c0 >= base + half) return;
     const int id = tok[t];
-    float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    if (id < 0 || id >= vocab) {
-        if (c == 0) atomicOr(status, KB_ST_BAD_TOKEN);
-    } else {
-        const TW* p = table + (size_t)id * E + c;
-        TW raw[8];
-        *(uint4*)raw = *(const uint4*)p;
-        if (sizeof(TW) == 4) *(uint4*)(raw + 4) = *(const uint4*)(p + 4);
+    const bool on = id >= 0 && id < vocab;
+    if (!on && c0 == 0) atomicOr(status, KB_ST_BAD_TOKEN);
+    const TW* p = table + (size_t)(on ? id : 0) * E;
+    float4 v[2];
 #pragma unroll
-        for (int i = 0; i < 8; i++) v[i] = scale == 1.0f ? kb_to_f<TW>(raw[i]) : kb_to_f<TW>(raw[i]) * scale;
+    for (int k = 0; k < 2; k++) {
+        const int c = c0 + half * k;
+        v[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (!on) continue;
+        if (sizeof(TW) == 2) {
+            const uint2 r = *(const uint2*)(p + c);
+            const float2 a = __bfloat1622float2(*(const __nv_bfloat162*)&r.x), b = __bfloat1622float2(*(const __nv_bfloat162*)&r.y);
+            v[k] = make_float4(a.x, a.y, b.x, b.y);
+        } else {
+            v[k] = *(const float4*)(p + c);
+        }
     }
-    float4* o = (float4*)(x + (size_t)t * E + c);
-    o[0] = make_float4(v[0], v[1], v[2], v[3]);
-    o[1] = make_float4(v[4], v[5], v[6], v[7]);
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        if (scale != 1.0f) v[k] = make_float4(v[k].x * scale, v[k].y * scale, v[k].z * scale, v[k].w * scale);
+        *(float4*)(x + (size_t)t * E + c0 + half * k) = v[k];
+    }
 }
 
 // x[t] = table[tok[t]] * scale (scale 1: the row as stored, the reference's embedding: kindi/nbq.cu:472-487)
@@ -70,7 +79,7 @@ extern "C" int kb_embed(const void* table, int wdtype, const int* tok, float* x,
                         float scale, int* status, cudaStream_t st) {
     if (T <= 0) return 0;
     if (E % 8 == 0 && ((uintptr_t)table & 15) == 0 && ((uintptr_t)x & 15) == 0) {
-        const dim3 grid(T, (E / 8 + 255) / 256);
+        const dim3 grid(T, (E + 2047) / 2048);
         if (wdtype == KB_F32) kb_launch(k_embed8<float>, grid, 256, 0, st, (const float*)table, tok, x, E, vocab, scale, status);
         else kb_launch(k_embed8<bf16>, grid, 256, 0, st, (const bf16*)table, tok, x, E, vocab, scale, status);
         KB_LAUNCH_RET();

@@ -703,3 +703,21 @@ def test_page_table_entries_from_pinned_memory(K):
         K.table_set(table, e, n)
         torch.cuda.synchronize()
         assert torch.equal(table, want)
+
+
+@pytest.mark.parametrize("E", [8, 40, 2048, 2056, 2060, 4104])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("scale", [1.0, 0.37])
+def test_embedding_rows_of_every_width(K, E, dtype, scale):
+    """rows in pieces of eight and rows that are not, tables that are aligned and one that is not, ids outside the table"""
+    g = torch.Generator(device="cuda").manual_seed(E)
+    store = torch.randn(50 * E + 8, device="cuda", generator=g).to(dtype)
+    tok = torch.tensor([0, 49, 7, 50, -1, 3, 2 ** 30], dtype=torch.int32, device="cuda")
+    for at in (0, 1):
+        table = store[at:at + 50 * E].view(50, E)
+        out, st = torch.full((7, E), 9.0, device="cuda"), _status()
+        K.embed(table, tok, out, st, scale)
+        want = torch.zeros(7, E, device="cuda")
+        ok = (tok >= 0) & (tok < 50)
+        want[ok] = table[tok[ok].long()].float() * torch.tensor(scale, device="cuda")
+        assert torch.equal(out, want) and int(st.item()) == K.ST_BAD_TOKEN
