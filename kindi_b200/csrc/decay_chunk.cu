@@ -8,10 +8,11 @@
 //   k_decay_out     the outputs of 64 tokens of a chunk for 64 columns of the state: the state's part, then the chunk's own
 //                   keys up to the tokens, tile by tile
 // No factor is ever divided out: every power of w has an exponent of at least zero.
-// What bounds it is the 32-bit FMA rate. The token-by-token form in its place held a column of the state per thread and made
-// three multiply-adds per state element and token with 12 warps on an SM: 289 us for 1777 tokens of 16 heads of 128 x 128.
+// What bounds it are the 32-bit multiply-adds and the phases between them (36 to 42 % of the FMA pipe, shared memory 66 to 69 %).
+// The form in its place held a column of the state per thread and made three multiply-adds per state element and token with 12
+// warps on an SM: 278 us for 1777 tokens of 16 heads of 128 x 128.
 // Here a thread makes 4 x 4 (4 x 8) outputs from 16-byte reads of shared memory, and a token costs two multiply-adds per
-// state element and 64 per element of its key and value: 148 us (43 + 14 + 92).
+// state element and 64 per element of its key and value: 133 us.
 #include "common.cuh"
 #include "mma_sync.cuh"
 
