@@ -1,0 +1,437 @@
+// Products of a decode step of few rows (up to 16): C = A W^T with every output finished by ONE block.
+//
+// Such a product reads its weights once and does next to no arithmetic: the memory bounds it, and beside the memory what
+// it costs to start and to end, because a decode step is a chain of a few dozen of them. The tensor-memory form
+// (gemm_tc.cu, "decode form") cuts the weights into tiles of 128 rows and splits K to fill the SMs; its partial planes
+// then need a consumer that adds them (the norm kernel between two products), and its blocks can request only their first
+// tile of weights before the kernel in front has ended. Here
+//   - block c takes the c-th of gridDim.x even stretches of the OUTPUTS over the whole of K, so that it can finish them:
+//     scale them, apply the gated unit, or add them into the residual stream, whose new values it also multiplies by the
+//     next norm's gains and squares (the next product divides by the root of the mean: a row's factor can wait until
+//     after the product). No planes, no norm kernel, no gated-unit kernel;
+//   - eight warps share K, each with a ring of 16 KB in shared memory that cp.async fills, 16 bytes a lane, rows exactly as the
+//     block's stretch has them (TMA boxes of 16 to 32 rows: 21.7 us for gate/up of 20992 x 2560 at one row, cp.async 18.2;
+//     straight into registers 36.6). 128 KB in flight an SM, all of it requested before the wait on the kernel in front:
+//     96 KB make a 3B-shaped step of eight layers 457 us, 128 KB 439. What an SM takes in bounds the rest of it, about 46
+//     bytes a nanosecond whether the weights come from memory or from the L2, so that asking for the next product's
+//     weights into the L2 made steps slower (439 -> 447 us with 64 KB a block), and so the activation rows, which every
+//     block reads whole, count like weights: at more than eight rows the tensor-memory form is the faster one;
+//   - a lane's 16 neighbouring elements of a row are its share of four m16n8k16 products (a product may take k in any order
+//     that both operands share);
+//   - the activation rows lie in shared memory (a bulk copy a row and warp) where they fit beside the next kernel's, else
+//     they come through the rings;
+//   - the warps' sums meet in shared memory and are added in the warps' order: the same bits on every run, and a row's
+//     bits do not depend on the other rows.
+// Measured (us a product behind another of its kind, memory-cold, tensor-memory form -> this, 1 | 8 rows): QKV 3584 x 2560
+// 6.2 -> 5.5 | 6.2 -> 6.2, output 2560 x 2560 5.2 -> 4.0 | 5.2 -> 5.6, gate/up 20.0 -> 18.2 | 21.7 -> 19.1, down 2560 x
+// 10496 11.6 -> 12.3 | 11.5 -> 12.8; a layer loses its two norm kernels (3.2 each). Steps of eight 3B-shaped layers: one
+// sequence of 517 507 -> 439, eight of 8191 677 -> 606; four layers of 512: 114 -> 87.
+// The reference's counterparts are its dp4a matrix-vector products (kindi/nbq.cu:266-296).
+#include "mma_sync.cuh"
+#include "sm100.cuh"
+
+#define GV_THREADS 256
+#define GV_WARPS (GV_THREADS / 32)
+#ifndef GV_RING
+#define GV_RING (16 * 1024)             // bytes of copies in flight a warp
+#endif
+#ifndef GV_ACT_SMEM
+#define GV_ACT_SMEM (48 * 1024)         // activation rows up to this size stay in shared memory
+#endif
+
+enum { GV_PLAIN = 0, GV_GLU = 1, GV_STREAM = 2 };
+
+struct GvArgs {
+    const bf16* A;              // [M][lda] activation rows
+    const bf16* W;              // [N][ldw]
+    int M, N, K, lda, ldw;
+    const float* ss;            // [M][ss_n] partial sums of squares of the rows of A, or null: A is taken as it is
+    int ss_n;
+    float inv_width, eps;       // the rows' factor is rsqrt(sum(ss) * inv_width + eps)
+    void* out;                  // GV_PLAIN: float [M][ldo]; GV_GLU: bf16 [M][ldo]; GV_STREAM: bf16 [M][ldo] = x * gain
+    int ldo;
+    float* x;                   // GV_STREAM: the stream [M][ldx], x += product (times branch_scale, where given)
+    int ldx;
+    const void* gain;           // GV_STREAM: the next norm's gains and the branch's scale per column (or null), of one type
+    const void* branch_scale;
+    int gain_f32;
+    float* ss_out;              // GV_STREAM: [M][gridDim.x] sums of squares of this block's part of the new x
+    int tile_out, tiles;        // outputs a tile, most tiles a block
+    int slots;                  // slots of a warp's ring that it can need
+    int act_off, ss_off, red_off, tp;   // shared memory: after the rings; a sum's pitch
+    int* status;
+    KbGate gate;
+};
+
+__device__ __forceinline__ float gv_gain(const void* g, int f32, int i) {
+    return f32 ? ((const float*)g)[i] : __bfloat162float(((const bf16*)g)[i]);
+}
+
+// a contiguous copy into shared memory: addresses and size multiples of 16 bytes
+__device__ __forceinline__ void gv_bulk(uint32_t dst, const void* src, int bytes, uint32_t bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
+}
+
+// G: groups of 8 rows of W a tile; NT: groups of 8 activation rows; SA: the activation rows stay in shared memory (else they come
+// through the ring, a K block beside the weights')
+template <int G, int NT, bool SA, int EPI>
+__global__ void __launch_bounds__(GV_THREADS, 2) k_gemv(const GvArgs a) {
+    extern __shared__ __align__(128) uint8_t gv_smem[];
+    __shared__ __align__(8) uint64_t s_bar[GV_WARPS];
+    kb_pdl_launch_now();
+    constexpr bool GLU = EPI == GV_GLU;
+    constexpr int MT = (G + 1) / 2;
+    constexpr int STAGE = (G + (SA ? 0 : NT)) * 1024;                // bytes: rows of 64 elements, 128 bytes each
+    constexpr int D = GV_RING / STAGE < 8 ? GV_RING / STAGE : 8;     // copies in flight a warp
+    static_assert(D >= 2, "a ring of one slot");
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+    const int n_out = GLU ? a.N >> 1 : a.N;
+    const int o0 = (int)(blockIdx.x * (unsigned)n_out / gridDim.x), o1 = (int)((blockIdx.x + 1) * (unsigned)n_out / gridDim.x);
+    const int n_o = o1 - o0, TO = a.tile_out, TP = a.tp;
+    const int n_kb = (a.K + 63) >> 6;
+    const int k0 = warp * n_kb / GV_WARPS, k1 = (warp + 1) * n_kb / GV_WARPS;
+    const int tiles = (n_o + TO - 1) / TO;
+    const int total = tiles * (k1 - k0);
+    // shared memory: the warps' rings, activation rows, the partial sums of squares, the warps' sums
+    const int pitch = ((a.K * 2 + 127) & ~127) + 16;                 // (rows 16 bytes apart modulo 128: no bank conflicts)
+    uint8_t* s_act = gv_smem + a.act_off;
+    uint8_t* s_ss = gv_smem + a.ss_off;
+    const int red_rows = GLU ? a.tiles * G * 8 : a.tiles * TO;
+    float* s_red = (float*)(gv_smem + a.red_off);
+    float* red = s_red + (size_t)warp * red_rows * TP;
+    const uint8_t* ring = gv_smem + warp * (a.slots * STAGE);
+    const uint32_t ring_u = smem_u32(ring), bar = smem_u32(&s_bar[warp]);
+
+    // copies: a lane brings 16 bytes (piece `pc` of a row's 128) of rows cr and cr + 4 of every group; a row's pieces are
+    // exchanged by its number, so that neither the copies nor the products' reads meet in a bank
+    const int cr = lane >> 3, pc = lane & 7;
+    const uint32_t cdst0 = cr * 128 + ((pc ^ cr) << 4), cdst1 = (cr + 4) * 128 + ((pc ^ (cr + 4)) << 4);
+    const bf16* src[G][2];                                           // (null: a row past the tile's)
+    int lt = 0, lk = k0;                                             // tile and K block of the next copy
+    auto rows_of_tile = [&](int t) {
+#pragma unroll
+        for (int i = 0; i < G; i++)
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const int r = (GLU ? i >> 1 : i) * 8 + cr + 4 * h, o = o0 + t * TO + r;
+                const int row = GLU ? (o >> 4) * 32 + (o & 15) + (i & 1) * 16 : o;
+                src[i][h] = r < TO && o < o1 ? a.W + (size_t)row * a.ldw + pc * 8 : nullptr;
+            }
+    };
+    auto load_w = [&](int slot) {
+        const bool ok = lk * 64 + pc * 8 < a.K;
+        const uint32_t dst = ring_u + slot * STAGE;
+#pragma unroll
+        for (int i = 0; i < G; i++) {
+            if (src[i][0]) cp_async16(dst + i * 1024 + cdst0, ok ? src[i][0] + lk * 64 : a.W, ok);
+            if (src[i][1]) cp_async16(dst + i * 1024 + cdst1, ok ? src[i][1] + lk * 64 : a.W, ok);
+        }
+    };
+    auto load_a = [&](int slot, int kb) {
+        if (!SA) {
+            const bool ok = kb * 64 + pc * 8 < a.K;
+            const uint32_t dst = ring_u + slot * STAGE + G * 1024;
+#pragma unroll
+            for (int n = 0; n < NT; n++) {
+                const int t = n * 8 + cr;
+                const bf16* p = a.A + (size_t)t * a.lda + kb * 64 + pc * 8;
+                if (t < a.M) cp_async16(dst + n * 1024 + cdst0, ok ? p : a.A, ok);
+                if (t + 4 < a.M) cp_async16(dst + n * 1024 + cdst1, ok ? p + (size_t)4 * a.lda : a.A, ok);
+            }
+        }
+    };
+    auto advance = [&]() {
+        if (++lk == k1) {
+            lk = k0;
+            rows_of_tile(++lt);
+        }
+    };
+    if (SA && lane == 0) {
+        mbar_init(bar, 1);
+        mbar_fence_init();
+    }
+    rows_of_tile(0);
+#pragma unroll
+    for (int d = 0; d < D; d++)
+    {
+        if (d < total) {
+            load_w(d);
+            advance();
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    if (SA && k1 == n_kb && k1 > k0)                                 // zeros from K to the end of its last block
+        for (int t = 0; t < a.M; t++)
+            for (int c = a.K * 2 + lane * 16; c < n_kb * 128; c += 512) *(uint4*)(s_act + t * pitch + c) = make_uint4(0, 0, 0, 0);
+    const int t_ep = warp, r_ep = o0 + lane;                         // GV_STREAM: this thread's first row and column
+    float gain_ep = 0.0f, scale_ep = 1.0f, x_ep[NT];
+    if (EPI == GV_STREAM && r_ep < o1) {
+        gain_ep = gv_gain(a.gain, a.gain_f32, r_ep);
+        if (a.branch_scale) scale_ep = gv_gain(a.branch_scale, a.gain_f32, r_ep);
+    }
+    __syncwarp();
+    kb_pdl_wait();
+    if (SA) {
+        // this warp's stretch of K of every row, a bulk copy a row
+        const int b0 = k0 * 128, nb = min(k1 * 128, a.K * 2) - b0;
+        if (k1 > k0) {
+            if (lane == 0) mbar_expect_tx(bar, a.M * nb);
+            __syncwarp();
+            if (lane < a.M) gv_bulk(smem_u32(s_act + lane * pitch + b0), (const uint8_t*)(a.A + (size_t)lane * a.lda) + b0, nb, bar);
+        }
+    } else {
+        int kb = k0;
+#pragma unroll
+        for (int d = 0; d < D; d++)
+            if (d < total) {
+                load_a(d, kb);
+                if (++kb == k1) kb = k0;
+            }
+    }
+    if (a.ss) {
+        const int n4 = a.ss_n >> 2;                                  // (ss_n is a multiple of 4: see the launcher)
+        for (int t = warp; t < a.M; t += GV_WARPS)
+            for (int c = lane; c < n4; c += 32) cp_async16(smem_u32(s_ss + ((size_t)t * n4 + c) * 16), a.ss + (size_t)t * a.ss_n + c * 4, true);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    if (EPI == GV_STREAM) {
+#pragma unroll
+        for (int n = 0; n < NT; n++)
+            x_ep[n] = r_ep < o1 && t_ep + 8 * n < a.M ? a.x[(size_t)(t_ep + 8 * n) * a.ldx + r_ep] : 0.0f;
+    }
+
+    float acc[MT][NT][4];
+#pragma unroll
+    for (int m = 0; m < MT; m++)
+#pragma unroll
+        for (int n = 0; n < NT; n++)
+#pragma unroll
+            for (int c = 0; c < 4; c++) acc[m][n][c] = 0.0f;
+    int ct = 0, ck = k0;                                             // tile and K block being multiplied
+    auto flush = [&]() {
+#pragma unroll
+        for (int m = 0; m < MT; m++)
+#pragma unroll
+            for (int n = 0; n < NT; n++)
+#pragma unroll
+                for (int c = 0; c < 4; c++) {
+                    const int r = (m * 2 + (c >> 1)) * 8 + g, t = n * 8 + q * 2 + (c & 1);
+                    const int row = GLU ? ct * G * 8 + r : ct * TO + r;
+                    if (m * 2 + (c >> 1) < G && (GLU || r < TO) && t < a.M) red[(size_t)row * TP + t] = acc[m][n][c];
+                    acc[m][n][c] = 0.0f;
+                }
+    };
+    bool good = true;
+    if (SA) {
+        if (k1 > k0) good = mbar_wait(bar, 0, a.status);
+    } else {
+        cp_async_wait_all();
+    }
+    if (__syncthreads_or(!good)) {
+        // (a wait ran out: the copies still under way, with a limit)
+        cp_async_wait_all();
+        if (!good) mbar_wait_ns(bar, 0, a.status, 10000000ull);
+        return;
+    }
+    const uint32_t rd0 = g * 128 + (((2 * q) ^ g) << 4), rd1 = g * 128 + (((2 * q + 1) ^ g) << 4);
+    int slot = 0, arow[NT];
+#pragma unroll
+    for (int n = 0; n < NT; n++) arow[n] = min(n * 8 + g, a.M - 1) * pitch + q * 32;
+    for (int s = 0; s < total; s++) {
+        if (SA || s >= D) asm volatile("cp.async.wait_group %0;" ::"n"(D - 1) : "memory");
+        __syncwarp();
+        const uint8_t* st = ring + slot * STAGE;
+        uint32_t wv[G][8], bx[NT][8];
+#pragma unroll
+        for (int i = 0; i < G; i++) {
+            *(uint4*)&wv[i][0] = *(const uint4*)(st + i * 1024 + rd0);
+            *(uint4*)&wv[i][4] = *(const uint4*)(st + i * 1024 + rd1);
+        }
+#pragma unroll
+        for (int n = 0; n < NT; n++) {
+            const uint8_t* p = SA ? s_act + arow[n] + ck * 128 : st + (G + n) * 1024 + rd0;
+            *(uint4*)&bx[n][0] = *(const uint4*)p;
+            *(uint4*)&bx[n][4] = SA ? *(const uint4*)(p + 16) : *(const uint4*)(st + (G + n) * 1024 + rd1);
+        }
+        __syncwarp();
+        if (s + D < total) {
+            load_w(slot);
+            load_a(slot, lk);
+            advance();
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        if (++slot == D) slot = 0;
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+#pragma unroll
+            for (int m = 0; m < MT; m++) {
+                constexpr int LAST = G - 1;
+                const bool odd = m * 2 + 1 > LAST;
+                const uint32_t fa[4] = {wv[m * 2][2 * j], odd ? 0u : wv[odd ? LAST : m * 2 + 1][2 * j], wv[m * 2][2 * j + 1],
+                                        odd ? 0u : wv[odd ? LAST : m * 2 + 1][2 * j + 1]};
+#pragma unroll
+                for (int n = 0; n < NT; n++) mma_bf16(acc[m][n], fa, bx[n][2 * j], bx[n][2 * j + 1]);
+            }
+        if (++ck == k1) {
+            flush();
+            ck = k0;
+            ct++;
+        }
+    }
+    if (k0 == k1)                                                    // (fewer K blocks than warps)
+        for (; ct < tiles; ct++) flush();
+    cp_async_wait_all();
+    __syncthreads();
+
+    // the warps' sums in their order; GV_STREAM: a warp a row, lanes over the block's columns; else the warps beyond the
+    // rows' number share a row's columns
+    const int wpr = EPI == GV_STREAM ? 1 : a.M <= 1 ? 8 : a.M <= 2 ? 4 : a.M <= 4 ? 2 : 1;
+    const int part = warp % wpr;
+    for (int t = warp / wpr, n = 0; t < a.M; t += GV_WARPS / wpr, n++) {
+        float f = 1.0f;
+        if (a.ss) {
+            float s = 0.0f;
+            for (int c = lane; c < a.ss_n; c += 32) s += ((const float*)s_ss)[(size_t)t * a.ss_n + c];
+            f = rsqrtf(kb_warp_sum(s) * a.inv_width + a.eps);
+        }
+        float sq = 0.0f;
+        for (int j = lane + 32 * part; j < n_o; j += 32 * wpr) {
+            if (EPI == GV_GLU) {
+                float gv = 0.0f, uv = 0.0f;
+#pragma unroll
+                for (int w = 0; w < GV_WARPS; w++) {
+                    const float* r = s_red + ((size_t)w * red_rows + (j >> 3) * 16 + (j & 7)) * TP + t;
+                    gv += r[0];
+                    uv += r[8 * TP];
+                }
+                ((bf16*)a.out)[(size_t)t * a.ldo + o0 + j] = __float2bfloat16_rn(kb_glu_fast(gv * f, uv * f, a.gate));
+            } else {
+                float v = 0.0f;
+#pragma unroll
+                for (int w = 0; w < GV_WARPS; w++) v += s_red[((size_t)w * red_rows + j) * TP + t];
+                if (a.ss) v *= f;
+                if (EPI == GV_PLAIN) {
+                    ((float*)a.out)[(size_t)t * a.ldo + o0 + j] = v;
+                } else {
+                    const bool first = j == lane;
+                    float* xp = a.x + (size_t)t * a.ldx + o0 + j;
+                    const float gn = first ? gain_ep : gv_gain(a.gain, a.gain_f32, o0 + j);
+                    if (a.branch_scale) v *= first ? scale_ep : gv_gain(a.branch_scale, a.gain_f32, o0 + j);
+                    float x0;
+                    if (first) {
+                        x0 = x_ep[0];
+                        if (NT > 1 && n == 1) x0 = x_ep[NT - 1];
+                    } else {
+                        x0 = *xp;
+                    }
+                    v = __fadd_rn(x0, v);
+                    *xp = v;
+                    ((bf16*)a.out)[(size_t)t * a.ldo + o0 + j] = __float2bfloat16_rn(v * gn);
+                    sq = fmaf(v, v, sq);
+                }
+            }
+        }
+        if (EPI == GV_STREAM) {
+            sq = kb_warp_sum(sq);
+            if (lane == 0) a.ss_out[(size_t)t * gridDim.x + blockIdx.x] = sq;
+        }
+    }
+}
+
+static int kb_sm_count() {
+    int dev = 0, n = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+    return n > 0 ? n : 148;
+}
+
+template <int G, int NT, bool SA, int EPI>
+static int gv_launch(const GvArgs& a, int smem, int grid, cudaStream_t st) {
+    auto kern = k_gemv<G, NT, SA, EPI>;
+    static char once_tag;
+    if (kb_first_use(&once_tag)) {
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);
+        if (e != cudaSuccess) return (int)e;
+    }
+    kb_launch(kern, grid, GV_THREADS, smem, st, a);
+    return (int)cudaGetLastError();
+}
+
+// blocks of a launch (and partial sums of squares a row): one an SM, rounded down to whole 16-byte pieces of partial sums
+extern "C" int kb_gemv_blocks() { return kb_sm_count() & ~3; }
+
+// how a launch cuts a block's outputs into tiles of even height, and its shared memory
+static int gv_plan(int M, int N, int K, int glu, int ss_n, int grid, GvArgs* a, int* G, int* sa, int* smem) {
+    const int n_out = glu ? N / 2 : N, block = (n_out + grid - 1) / grid, nt = M <= 8 ? 1 : 2;
+    const int pitch = ((K * 2 + 127) & ~127) + 16;
+    *sa = (long long)M * pitch <= GV_ACT_SMEM;
+    if (glu) {
+        *G = 2;
+        a->tile_out = 8;
+        a->tiles = (block + 7) / 8;
+    } else {
+        a->tiles = (block + 31) / 32;
+        a->tile_out = (block + a->tiles - 1) / a->tiles;
+        *G = (a->tile_out + 7) / 8;
+    }
+    const int stage = (*G + (*sa ? 0 : nt)) * 1024, depth = GV_RING / stage < 8 ? GV_RING / stage : 8;
+    const long long red_rows = (long long)a->tiles * (glu ? *G * 8 : a->tile_out);
+    a->tp = M | 1;
+    const int most = a->tiles * ((((K + 63) >> 6) + GV_WARPS - 1) / GV_WARPS);        // (a warp's copies: the slots it can need)
+    a->slots = most < depth ? most : depth;
+    a->act_off = GV_WARPS * a->slots * stage;
+    a->ss_off = a->act_off + (*sa ? M * pitch : 0);
+    a->red_off = a->ss_off + M * ss_n * 4;
+    const long long all = a->red_off + GV_WARPS * red_rows * a->tp * 4;
+    *smem = (int)(all < (1 << 30) ? all : 1 << 30);
+    return *smem <= 224 * 1024;
+}
+
+// 1 when kb_gemv takes the product: few rows, K in pieces of 16, sums that fit the shared memory
+extern "C" int kb_gemv_takes(int M, int N, int K, int lda, int ldw, int glu, int ss_n) {
+    if (M < 1 || M > 16 || N < 1 || K < 16 || (K & 15) || (lda & 7) || (ldw & 7) || (glu && (N & 31)) || (ss_n & 3)) return 0;
+    GvArgs a;
+    int G, sa, smem;
+    return gv_plan(M, N, K, glu, ss_n, kb_gemv_blocks(), &a, &G, &sa, &smem);
+}
+
+// C = A W^T for up to 16 rows. epi 0: out float [M][ldo]; epi 1: out bf16 [M][ldo] = the gated unit, W in groups of 16
+// gate rows and the 16 up rows of the same outputs; epi 2: x [M][ldx] += C (times branch_scale per column), out bf16 =
+// new x * gain, ss_out [M][kb_gemv_blocks()] = partial sums of squares of the new x. ss (or null) [M][ss_n]: the rows of A
+// are multiplied by rsqrt(sum(ss) / width + eps) (after the product).
+extern "C" int kb_gemv(const void* A, const void* W, int M, int N, int K, int lda, int ldw, const float* ss, int ss_n, int width,
+                       float eps, int epi, void* out, int ldo, int act, float act_lim, float act_alpha, float* x, int ldx,
+                       const void* gain, const void* branch_scale, int gain_f32, float* ss_out, int* status, cudaStream_t st) {
+    if (!ss) ss_n = 0;
+    if (epi < 0 || epi > 2 || !kb_gemv_takes(M, N, K, lda, ldw, epi == GV_GLU, ss_n)) return (int)cudaErrorInvalidValue;
+    if (((uintptr_t)A & 15) || ((uintptr_t)W & 15) || ((uintptr_t)ss & 15) || !status) return (int)cudaErrorInvalidValue;
+    if (epi == GV_STREAM && (!x || !gain || !ss_out)) return (int)cudaErrorInvalidValue;
+    GvArgs a = {};
+    a.A = (const bf16*)A; a.W = (const bf16*)W;
+    a.M = M; a.N = N; a.K = K; a.lda = lda; a.ldw = ldw;
+    a.ss = ss; a.ss_n = ss_n; a.inv_width = width > 0 ? 1.0f / (float)width : 0.0f; a.eps = eps;
+    a.out = out; a.ldo = ldo; a.x = x; a.ldx = ldx; a.gain = gain; a.branch_scale = branch_scale; a.gain_f32 = gain_f32;
+    a.ss_out = ss_out;
+    a.status = status;
+    a.gate = kb_gate_of(act, act_lim, act_alpha);
+    const int grid = kb_gemv_blocks();
+    int G, sa, smem;
+    if (!gv_plan(M, N, K, epi == GV_GLU, ss_n, grid, &a, &G, &sa, &smem)) return (int)cudaErrorInvalidValue;
+#define GV_GO(EPI_, G_)                                                                                            \
+    if (epi == EPI_ && G == G_) {                                                                                  \
+        if (sa) return M > 8 ? gv_launch<G_, 2, true, EPI_>(a, smem, grid, st) : gv_launch<G_, 1, true, EPI_>(a, smem, grid, st); \
+        return M > 8 ? gv_launch<G_, 2, false, EPI_>(a, smem, grid, st) : gv_launch<G_, 1, false, EPI_>(a, smem, grid, st);       \
+    }
+    GV_GO(GV_PLAIN, 1)
+    GV_GO(GV_PLAIN, 2)
+    GV_GO(GV_PLAIN, 3)
+    GV_GO(GV_PLAIN, 4)
+    GV_GO(GV_STREAM, 1)
+    GV_GO(GV_STREAM, 2)
+    GV_GO(GV_STREAM, 3)
+    GV_GO(GV_STREAM, 4)
+    GV_GO(GV_GLU, 2)
+#undef GV_GO
+    return (int)cudaErrorInvalidValue;
+}

@@ -150,6 +150,17 @@ def _prefill_product(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, status
                 post=post)
 
 
+# up to here a product may go through the kernel whose blocks finish their outputs (16 rows: its down product of 2560 x 10496
+# takes 15.9 us, the tensor-memory form 11.6: every block reads all activation rows)
+GEMV_ROWS = 8
+
+
+def gemv_ok(m: int, lda: int, w: torch.Tensor, glu: bool = False, squares: bool = False) -> bool:
+    """whether a product of ``m`` rows (of row stride ``lda``) with ``w`` goes through ``K.gemv``"""
+    return (m <= GEMV_ROWS and w.dtype == torch.bfloat16 and w.dim() == 2 and w.stride(1) == 1 and w.data_ptr() % 16 == 0
+            and K.gemv_takes(m, w.shape[0], w.shape[1], lda, w.stride(0), glu, squares))
+
+
 def gemm_rows(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, status: torch.Tensor) -> bool:
     if not _tc_ok(a, w) or not out.is_contiguous():
         return False

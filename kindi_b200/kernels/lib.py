@@ -136,6 +136,10 @@ _SIGS = {
     "kb_gemm_tc": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
                    c_longlong, c_void_p, c_void_p, c_int, c_int, c_float, c_float, c_void_p, c_int, c_int],
     "kb_gemm_tc_splits": [c_int, c_int],
+    "kb_gemv_blocks": [],
+    "kb_gemv_takes": [c_int, c_int, c_int, c_int, c_int, c_int, c_int],
+    "kb_gemv": [c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int, c_int, c_float, c_int, c_void_p, c_int,
+                c_int, c_float, c_float, c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p],
     "kb_rope_table_min_rows": [],
     "kb_gemm_pair": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p,
                      c_void_p, c_int, c_void_p, c_void_p, c_float, c_float, c_void_p, c_int],
@@ -208,7 +212,8 @@ def load(verbose: bool = True):
 _timing = None
 
 # where an entry point's product sizes stand among its arguments (N, K), for the label of a timed launch
-_GEMM_NK = {"kb_gemm_tc": (5, 6), "kb_gemm_pair": (5, 6), "kb_gemm_simt": (7, 8), "kb_gemm_swiglu_decode": (4, 5)}
+_GEMM_NK = {"kb_gemm_tc": (5, 6), "kb_gemm_pair": (5, 6), "kb_gemm_simt": (7, 8), "kb_gemm_swiglu_decode": (4, 5),
+            "kb_gemv": (3, 4)}
 
 
 class KernelTiming:
@@ -223,7 +228,7 @@ class KernelTiming:
 
     def __getattr__(self, name):                       # stands in for the library while timing is on
         fn = getattr(_lib, name)
-        if not name.startswith("kb_") or name in ("kb_set_pdl", "kb_gemm_tc_splits", "kb_rope_table_min_rows",
+        if not name.startswith("kb_") or name in ("kb_set_pdl", "kb_gemm_tc_splits", "kb_rope_table_min_rows", "kb_gemv_blocks", "kb_gemv_takes",
                                                   "kb_moe_gemm_tile", "kb_moe_gemm_tc_tile", "kb_scan_run",
                                                   "kb_wkv_run"):
             return fn
@@ -973,6 +978,53 @@ def gemm_tc(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, *, swap: bool, 
     _check(load().kb_gemm_tc(_p(a), _p(w), _p(out), dt(out), M, N, K, a.stride(0), w.stride(0), ldc, 1 if swap else 0,
                              bn, splits, stride, _p(status), _stream(), GATE_ACT[act] if swiglu else 0, mt,
                              *_gate_params(act, act_params), _p(bias), pact, int(group_rows)), "gemm_tc")
+
+
+@functools.lru_cache(maxsize=1)
+def gemv_blocks() -> int:
+    """blocks of a ``gemv`` launch: partial sums of squares a row that its stream form writes"""
+    return int(load().kb_gemv_blocks())
+
+
+@functools.lru_cache(maxsize=4096)
+def gemv_takes(m: int, n: int, k: int, lda: int, ldw: int, glu: bool, squares: bool) -> bool:
+    """whether ``gemv`` takes a product of these sizes (``squares``: of rows whose norm is still to be divided out)"""
+    return bool(load().kb_gemv_takes(m, n, k, lda, ldw, 1 if glu else 0, gemv_blocks() if squares else 0))
+
+
+def gemv(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, status: torch.Tensor, *, squares: Optional[torch.Tensor] = None, width: int = 0,
+         eps: float = 0.0, glu: bool = False, act: str = "silu", act_params=None, x: Optional[torch.Tensor] = None,
+         gain: Optional[torch.Tensor] = None, branch_scale: Optional[torch.Tensor] = None,
+         squares_out: Optional[torch.Tensor] = None) -> None:
+    """a[M, K] @ w[N, K]^T of up to 16 bf16 rows, every output finished by one block. ``squares`` (float32 [M,
+    gemv_blocks()]): partial sums of squares of the rows, which are multiplied by rsqrt(sum / width + eps) after the product.
+    ``out`` is float32 [M, N]; with ``glu`` the bf16 gated unit [M, N / 2] (w in groups of 16 gate rows and the 16 up rows
+    of the same outputs); with ``x`` (float32 [M, N], updated in place) x += product (times ``branch_scale`` per column),
+    ``out`` (bf16) = new x * ``gain`` and ``squares_out`` the partial sums of squares of the new x"""
+    _need_cuda(a, w, out, squares, x, gain, branch_scale, squares_out)
+    M, k = a.shape
+    N = w.shape[0]
+    assert a.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and w.shape[1] == k
+    assert a.stride(1) == 1 and w.stride(1) == 1 and out.stride(1) == 1
+    epi = 2 if x is not None else 1 if glu else 0
+    if epi == 0:
+        assert out.shape == (M, N) and out.dtype == torch.float32
+    elif epi == 1:
+        assert out.shape == (M, N // 2) and out.dtype == torch.bfloat16
+    else:
+        assert out.shape == (M, N) and out.dtype == torch.bfloat16 and x.shape == (M, N) and x.dtype == torch.float32
+        assert x.stride(1) == 1 and gain.numel() == N and gain.is_contiguous()
+        assert squares_out.shape == (M, gemv_blocks()) and squares_out.dtype == torch.float32 and squares_out.is_contiguous()
+        assert branch_scale is None or (branch_scale.dtype == gain.dtype and branch_scale.numel() == N
+                                        and branch_scale.is_contiguous())
+    n_sq = 0
+    if squares is not None:
+        assert squares.dtype == torch.float32 and squares.is_contiguous() and squares.shape[0] == M
+        n_sq = squares.shape[1]
+    _check(load().kb_gemv(_p(a), _p(w), M, N, k, a.stride(0), w.stride(0), _p(squares), n_sq, int(width), float(eps), epi,
+                          _p(out), out.stride(0), GATE_ACT[act] if glu else 0, *_gate_params(act, act_params), _p(x),
+                          x.stride(0) if x is not None else 0, _p(gain), _p(branch_scale),
+                          1 if gain is not None and dt(gain) == F32 else 0, _p(squares_out), _p(status), _stream()), "gemv")
 
 
 def gemm_pair(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, *, bn: int, status: torch.Tensor,

@@ -34,9 +34,38 @@ def planes(ctx, a: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
     return out
 
 
+def takes_scaled(ctx, w: torch.Tensor, glu: bool = False) -> bool:
+    """whether a product of the step's rows with ``w`` may be given ``ScaledRows`` (rows whose norm is divided out after the
+    product): decode-sized steps of the serving kernels"""
+    return ctx.fast and fast.gemv_ok(ctx.T, w.shape[1], w, glu, True)
+
+
+def branch(ctx, a: torch.Tensor, w: torch.Tensor):
+    """the branch ``a @ w^T``: launched by the norm that adds it, so that a decode-sized step can finish the add and the
+    norm's gains inside the product"""
+    from ..parts.base import LazyBranch
+    return LazyBranch(ctx, a, w)
+
+
+def stream_product(ctx, a: torch.Tensor, w: torch.Tensor, x: torch.Tensor, gain: torch.Tensor, branch_scale):
+    """x += a @ w^T (times ``branch_scale`` per column) and, from the new x, (x * gain in bf16, partial sums of its squares);
+    None, with nothing launched, where no kernel takes the shape"""
+    if not (ctx.fast and a.dtype == torch.bfloat16 and a.stride(1) == 1 and a.data_ptr() % 16 == 0
+            and x.is_contiguous() and fast.gemv_ok(a.shape[0], a.stride(0), w)):
+        return None
+    y = torch.empty(x.shape, dtype=torch.bfloat16, device=x.device)
+    squares = torch.empty((x.shape[0], K.gemv_blocks()), dtype=torch.float32, device=x.device)
+    K.gemv(a, w, y, ctx.status, x=x, gain=gain, branch_scale=branch_scale, squares_out=squares)
+    return y, squares
+
+
 def rows_or_planes(ctx, a: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype) -> torch.Tensor:
     """the product for a consumer that takes either form: 32-bit planes when the step is small (so that K can be
-    split), else rows in out_dtype"""
+    split), else rows in out_dtype. ``a`` may be ``ScaledRows`` where ``takes_scaled`` says so"""
+    if not isinstance(a, torch.Tensor):
+        out = torch.empty((1, a.shape[0], w.shape[0]), dtype=torch.float32, device=a.device)
+        K.gemv(a.rows, w, out[0], ctx.status, squares=a.squares, width=a.shape[1], eps=a.eps)
+        return out
     if ctx.fast and fast.wants_planes(a, w):
         p = fast.gemm_planes(a, w, ctx.status)
         if p is not None:
@@ -75,8 +104,11 @@ def gate_up_swiglu(ctx, y: torch.Tensor, wgu: torch.Tensor, group: int, f: int, 
                    act: str = "silu") -> torch.Tensor:
     """``act(g) * u`` (``[M, F]`` in out_dtype; ``act`` silu or gelu_tanh) with ``[g | u] = y @ wgu^T``, ``wgu`` as
     ``join_gate_up`` made it: inside the product where a tensor-core kernel takes the shape, else the product followed
-    by the SwiGLU kernel"""
+    by the SwiGLU kernel. ``y`` may be ``ScaledRows`` where ``takes_scaled`` says so"""
     h = torch.empty((y.shape[0], f), dtype=out_dtype, device=y.device)
+    if not isinstance(y, torch.Tensor):
+        K.gemv(y.rows, wgu, h, ctx.status, squares=y.squares, width=y.shape[1], eps=y.eps, glu=True, act=act)
+        return h
     if ctx.fast and group == GATE_UP_GROUP and (fast.gemm_swiglu_decode(y, wgu, h, ctx.status, act)
                                                 or fast.gemm_swiglu_rows(y, wgu, h, ctx.status, act)):
         return h

@@ -158,6 +158,9 @@ class CausalSelfAttention(Mixer):
                             _pad_heads(weights(qkn["k"]), self.nkv, self.qk_dim, self.hd).contiguous(),
                             float(qkn["eps"]), self.nh * self.qk_dim, self.nkv * self.qk_dim)
 
+    def takes_scaled_rows(self, ctx: StepContext) -> bool:
+        return L.takes_scaled(ctx, self.wqkv)
+
     def forward(self, ctx: StepContext, y: torch.Tensor) -> Branch:
         nh, nkv, hd = self.nh, self.nkv, self.hd
         entry = ctx.entry
@@ -180,7 +183,7 @@ class CausalSelfAttention(Mixer):
         if plain and not reads_other and A.attention_from_planes(ctx, qkv, att, nh, nkv, hd, self.scale, self.window,
                                                                  self.position.rotation(), pool, table, n_pages):
             # a small decode step of the serving kernels: the attention kernel summed the planes, rotated and stored
-            return Branch(L.planes(ctx, att, self.wo))
+            return L.branch(ctx, att, self.wo)
         # the position encoding sums 32-bit planes, encodes and writes the queries out as rows (rows are encoded in
         # place) and stores keys and values; then attention over the cache
         q = qkv if qkv.dim() == 2 else torch.empty((ctx.T, n_q), dtype=self.dtype, device=y.device)
@@ -190,7 +193,7 @@ class CausalSelfAttention(Mixer):
             self.position.encode_and_store(ctx, qkv, q, nh, store_kv, hd, pool, table, n_pages, qk_norm=self.qk_norm)
         A.attention(ctx, q, att, nh, nkv, hd, self.scale, self.window, pool, table, n_pages,
                     keep_first=self.keep_first)
-        return Branch(L.planes(ctx, att, self.wo))
+        return L.branch(ctx, att, self.wo)
 
     def _forward_sink_gate(self, ctx: StepContext, y: torch.Tensor, reads_other: bool) -> Branch:
         """the same steps for a layer with a sink in its softmax or a gate on its output: one product for
@@ -222,7 +225,7 @@ class CausalSelfAttention(Mixer):
                             keep_first=self.keep_first, sink=self.sink, gate=gate)
         if gate is not None and not fused:
             K.gate_mul(att, gate, att)
-        return Branch(L.planes(ctx, att, self.wo))
+        return L.branch(ctx, att, self.wo)
 
     def bytes_read(self) -> int:
         return sum(w.numel() * w.element_size() for w in (self.wqkv, self.wo))

@@ -105,6 +105,42 @@ class Branch:
         return Branch(torch.cat([self.parts, plane], dim=0), self.scale, None, self.norm)
 
 
+class LazyBranch(Branch):
+    """a branch that is one product ``a @ w^T`` nothing has launched yet: ``parts`` launches it as 32-bit planes when it is
+    asked for, unless the norm that adds the branch runs the product itself and finishes the add inside it
+    (``Norm.add_norm_scaled``)"""
+
+    def __init__(self, ctx: StepContext, a: torch.Tensor, w: torch.Tensor):
+        self.ctx, self.a, self.w = ctx, a, w
+        self.scale = self.bias = self.norm = self._parts = None
+
+    @property
+    def parts(self) -> torch.Tensor:
+        if self._parts is None:
+            from ..kernels import linear as L
+            self._parts = L.planes(self.ctx, self.a, self.w)
+        return self._parts
+
+
+@dataclass
+class ScaledRows:
+    """the rows a norm hands to a product that takes them before their division: row t of the norm's output is ``rows[t] *
+    rsqrt(sum(squares[t]) / width + eps)`` with ``rows`` (run dtype ``[T, width]``) the stream times the gains and
+    ``squares`` (float32) partial sums of squares of the stream's row"""
+
+    rows: torch.Tensor
+    squares: torch.Tensor
+    eps: float
+
+    @property
+    def shape(self):
+        return self.rows.shape
+
+    @property
+    def device(self):
+        return self.rows.device
+
+
 # ----------------------------------------------------------------------------- tensors by name
 class WeightView:
     """the tensors of one prefix (``model.layers.3.``): parts ask for them by their own suffixes"""
@@ -160,6 +196,11 @@ class Norm(Part):
         """``x`` (32-bit ``[T, width]``) += pending branch (written back unless ``rows`` is given); returns the
         normalised rows in the run dtype: all ``T`` rows, or the rows listed in ``rows`` (int32)"""
         raise NotImplementedError
+
+    def add_norm_scaled(self, ctx: StepContext, x: torch.Tensor, pending: Optional[Branch]) -> Optional["ScaledRows"]:
+        """the same for a reader that takes ``ScaledRows`` (``takes_scaled_rows``), where the norm can run the pending
+        branch's product itself and leave its rows undivided; None, with nothing launched: it cannot"""
+        return None
 
 
 class Embedding(Part):
@@ -229,12 +270,20 @@ class Mixer(Part):
         by ``ctx.cache.state_view(entry, self.state_base + k)`` in the order they stand here"""
         return None
 
+    def takes_scaled_rows(self, ctx: StepContext) -> bool:
+        """whether ``forward`` takes ``ScaledRows`` in the place of the normalised rows in this step"""
+        return False
+
     def forward(self, ctx: StepContext, y: torch.Tensor) -> Branch:
         raise NotImplementedError
 
 
 class FeedForward(Part):
     category = "feed_forward"
+
+    def takes_scaled_rows(self, ctx: StepContext) -> bool:
+        """whether ``forward`` takes ``ScaledRows`` in the place of the normalised rows in this step"""
+        return False
 
     def forward(self, ctx: StepContext, y: torch.Tensor) -> Branch:
         raise NotImplementedError

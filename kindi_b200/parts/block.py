@@ -93,13 +93,22 @@ class PreNormBlock(Block):
     def _parts(self):
         return [p for p in (self.norm1, self.mixer, self.norm2, self.feed_forward) if p is not None]
 
+    @staticmethod
+    def _norm(ctx: StepContext, norm, reader, x, pending: Optional[Branch]):
+        """the rows that ``reader`` reads: undivided, out of the pending branch's own product, where all three allow it"""
+        if pending is not None and reader.takes_scaled_rows(ctx):
+            y = norm.add_norm_scaled(ctx, x, pending)
+            if y is not None:
+                return y
+        return norm.add_norm(ctx, x, pending)
+
     def forward(self, ctx: StepContext, x, pending: Optional[Branch]) -> Optional[Branch]:
-        y = self.norm1.add_norm(ctx, x, pending)
+        y = self._norm(ctx, self.norm1, self.mixer, x, pending)
         pending = self.mixer.forward(ctx, y).with_bias_plane()
         pending.scale = self.scale1
         if self.feed_forward is None:
             return pending
-        y = self.norm2.add_norm(ctx, x, pending)
+        y = self._norm(ctx, self.norm2, self.feed_forward, x, pending)
         pending = self.feed_forward.forward(ctx, y)
         pending.scale = self.scale2
         return pending

@@ -48,9 +48,12 @@ class SwiGLU(FeedForward):
         self.wgu, self.group = L.join_gate_up(g, u)
         self.wd = weights(n["down"])
 
+    def takes_scaled_rows(self, ctx: StepContext) -> bool:
+        return self.group == L.GATE_UP_GROUP and L.takes_scaled(ctx, self.wgu, glu=True)
+
     def forward(self, ctx: StepContext, y: torch.Tensor) -> Branch:
         h = L.gate_up_swiglu(ctx, y, self.wgu, self.group, self.f, self.dtype, self.act)
-        return Branch(L.planes(ctx, h, self.wd))
+        return L.branch(ctx, h, self.wd)
 
     def bytes_read(self) -> int:
         return sum(w.numel() * w.element_size() for w in (self.wgu, self.wd))

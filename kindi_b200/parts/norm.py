@@ -15,7 +15,8 @@ import torch
 from ..config.registry import register_part
 from ..config.spec import PartSpec
 from ..kernels import lib as K
-from .base import Branch, Norm, StepContext, WeightView
+from ..kernels import linear as L
+from .base import Branch, LazyBranch, Norm, ScaledRows, StepContext, WeightView
 
 
 class RMSNorm(Norm):
@@ -59,6 +60,15 @@ class RMSNorm(Norm):
         K.add_rmsnorm(x, None if pending is None else pending.parts, self.weight, self.eps, y, rows,
                       write_back=rows is None and pending is not None, status=ctx.status, branch_scale=scale)
         return y
+
+    def add_norm_scaled(self, ctx: StepContext, x, pending: Optional[Branch]) -> Optional[ScaledRows]:
+        if not isinstance(pending, LazyBranch) or pending.bias is not None or pending.norm is not None:
+            return None
+        scale = pending.scale
+        if scale is not None and scale.dtype != self.weight.dtype:
+            scale = scale.to(self.weight.dtype)
+        made = L.stream_product(ctx, pending.a, pending.w, x, self.weight, scale)
+        return None if made is None else ScaledRows(made[0], made[1], self.eps)
 
     def bytes_read(self) -> int:
         return self.weight.numel() * self.weight.element_size()

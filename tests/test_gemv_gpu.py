@@ -1,0 +1,93 @@
+"""Products of up to 16 rows whose blocks finish their outputs (``gemv.cu``), against the product in 64 bits."""
+import pytest
+import torch
+
+from kindi_b200.kernels import lib as K
+
+pytestmark = pytest.mark.gpu
+
+# rows, outputs, K: one and several groups of 8 rows a block and tile, fewer outputs than blocks, K with a partial block and with
+# fewer blocks than warps, activations in shared memory and in registers
+SIZES = [(1, 512, 512), (8, 3584, 2560), (9, 2560, 10496), (16, 2560, 2560), (3, 100, 80), (2, 2560, 1408), (7, 6144, 16),
+         (16, 1000, 9008), (5, 5120, 13824), (1, 4099, 2832)]
+
+
+def ST():
+    return torch.zeros(1, dtype=torch.int32, device="cuda")
+
+
+def _data(m, n, k, seed=0):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    a = torch.randn(m, k, device="cuda", generator=g).bfloat16()
+    w = (torch.randn(n, k, device="cuda", generator=g) * 0.05).bfloat16()
+    return a, w
+
+
+def _close(got, want, scale):
+    # 32-bit sums of K exact products: K 2^-24 of the sum of magnitudes at the very most, in practice its root
+    err = ((got.double() - want).abs() / scale).max().item()
+    assert err < 2e-6, err
+
+
+@pytest.mark.parametrize("m,n,k", SIZES)
+@pytest.mark.parametrize("squares", [False, True])
+def test_plain_product(m, n, k, squares):
+    a, w = _data(m, n, k)
+    out = torch.full((m, n), float("nan"), device="cuda")
+    f = torch.ones(m, 1, dtype=torch.float64, device="cuda")
+    more = {}
+    if squares:
+        sq = torch.rand(m, K.gemv_blocks(), device="cuda")
+        f = 1.0 / (sq.double().sum(1, keepdim=True) / 77 + 1e-5).sqrt()
+        more = dict(squares=sq, width=77, eps=1e-5)
+    K.gemv(a, w, out, ST(), **more)
+    want = a.double() @ w.double().T
+    _close(out, want * f, a.double().abs() @ w.double().abs().T * f)
+
+
+@pytest.mark.parametrize("m,f,k", [(1, 1408, 512), (8, 10496, 2560), (16, 2816, 1024), (3, 16, 96), (12, 96, 5120)])
+def test_gated_unit(m, f, k):
+    a, w = _data(m, 2 * f, k)
+    sq = torch.rand(m, K.gemv_blocks(), device="cuda")
+    out = torch.zeros(m, f, device="cuda", dtype=torch.bfloat16)
+    K.gemv(a, w, out, ST(), squares=sq, width=k, eps=1e-5, glu=True)
+    p = (a.double() @ w.double().T / (sq.double().sum(1, keepdim=True) / k + 1e-5).sqrt()).view(m, f // 16, 2, 16)
+    gate, up = p[:, :, 0].reshape(m, f), p[:, :, 1].reshape(m, f)
+    want = gate / (1.0 + (-gate).exp()) * up
+    assert ((out.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-4 * want.abs().max()).all()
+
+
+@pytest.mark.parametrize("m,n,k", SIZES)
+@pytest.mark.parametrize("gain_dtype,scaled", [(torch.bfloat16, False), (torch.float32, True)])
+def test_stream(m, n, k, gain_dtype, scaled):
+    a, w = _data(m, n, k, 1)
+    x = torch.randn(m, n, device="cuda")
+    gain = (1.0 + 0.1 * torch.randn(n, device="cuda")).to(gain_dtype)
+    ls = (1.0 + 0.1 * torch.randn(n, device="cuda")).to(gain_dtype) if scaled else None
+    want = x.double() + a.double() @ w.double().T * (1.0 if ls is None else ls.double())
+    mag = x.double().abs() + a.double().abs() @ w.double().abs().T * 1.5
+    y = torch.zeros(m, n, device="cuda", dtype=torch.bfloat16)
+    sq = torch.full((m, K.gemv_blocks()), float("nan"), device="cuda")
+    K.gemv(a, w, y, ST(), x=x, gain=gain, branch_scale=ls, squares_out=sq)
+    _close(x, want, mag)
+    assert torch.equal(y, (x * gain.float()).bfloat16())
+    ss = (x.double() ** 2).sum(1)
+    assert ((sq.double().sum(1) - ss).abs() < 1e-5 * ss).all()
+
+
+def test_rows_do_not_depend_on_one_another():
+    a, w = _data(8, 3584, 2560)
+    out, one = torch.empty(8, 3584, device="cuda"), torch.empty(1, 3584, device="cuda")
+    K.gemv(a, w, out, ST())
+    for i in (0, 5):
+        K.gemv(a[i:i + 1].contiguous(), w, one, ST())
+        assert torch.equal(one[0], out[i])
+
+
+def test_what_it_does_not_take():
+    takes = K.gemv_takes
+    assert not takes(17, 512, 512, 512, 512, False, False)       # rows
+    assert not takes(4, 512, 520, 520, 520, False, False)        # K in pieces of 8
+    assert not takes(4, 512, 512, 512, 516, False, False)        # weight rows that 16-byte copies cannot take
+    assert not takes(4, 520, 512, 512, 512, True, False)         # gate and up rows not in groups of 16
+    assert not takes(8, 166144, 2560, 2560, 2560, False, False)  # more outputs a block than its sums have room for
