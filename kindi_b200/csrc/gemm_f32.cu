@@ -116,31 +116,52 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN)) k_gemm_f32(const float*
     }
 }
 
+static int f32_sms() {
+    static int sms = 0;
+    if (!sms) {
+        int dev = 0;
+        cudaGetDevice(&dev);
+        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
+    }
+    return sms;
+}
+// The shared memory to ask for, so that an SM takes no more than its even share of a grid of few blocks. A product's blocks are
+// placed while the kernel in front still runs, and then two come to lie on one SM while another stays empty: 514 x 1024
+// outputs, 144 blocks, took 77 us behind another product and 40 where no two share an SM; over K = 2816 205 and 104, 1200 x
+// 1024 (608 blocks) 92 and 79.
+static size_t f32_smem(int need, long long units) {
+    const long long share = (units + f32_sms() - 1) / f32_sms();
+    if (share > 10) return need;
+    const int ask = (int)(227 * 1024 / (share + 1)) + 1024;
+    return ask > need ? ask : need;
+}
+
 template <int BM, int BN, int TM, int TN, int BK, int STAGES>
 static int launch_f32(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw, int ldc,
                       cudaStream_t st) {
     using S = F32Tile<BM, BN, TM, TN, BK, STAGES>;
     auto kern = k_gemm_f32<BM, BN, TM, TN, BK, STAGES>;
     static char once_tag;
-    if (S::SMEM > 48 * 1024 && kb_first_use(&once_tag)) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::SMEM);
+    if (kb_first_use(&once_tag)) {
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 1024);
         if (e != cudaSuccess) return (int)e;
     }
-    kb_launch(kern, dim3((N + BN - 1) / BN, (M + BM - 1) / BM), S::THREADS, S::SMEM, st, A, W, C, M, N, K, lda, ldw, ldc);
+    const dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
+    kb_launch(kern, grid, S::THREADS, f32_smem(S::SMEM, (long long)grid.x * grid.y), st, A, W, C, M, N, K, lda, ldw, ldc);
     KB_LAUNCH_RET();
 }
 
 // The tiles, and what a product over 1024 K elements takes on them, in microseconds, by the rounds of units (ceil(units / SMs));
-// measured at 1 to 2048 rows of 8 to 32768 columns over K = 256, 1024 and 4096. Within the first round a lone unit on its SM
-// takes `few` while up to six tenths of the SMs have one, `full` beyond: the thin tiles fetch the most for a product and share
-// the way from the L2. The tile that this picks is 1.0 % slower than the best of the eight on average over those 440 products
-// (costs of a lone and of an added unit, with a charge from 90 units on: 3.8 %). 514 x 1024 outputs over K = 1024 take 73 us in
-// tiles of 64 x 128, 42 in 64 x 64 (144 units, chosen), 44 in 32 x 64, 59 in 32 x 32; 514 x 256 71, 39, 24 and 19 (chosen).
+// measured at 60 to 1200 rows of 1024 to 32768 columns with every SM held to its even share of a grid (f32_smem). Within the
+// first round a lone unit on its SM takes `few` while up to six tenths of the SMs have one, `full` beyond. 514 x 1024 outputs
+// over K = 1024 take 72 us in tiles of 64 x 128, 40 in 64 x 64 (144 units, chosen), 41 in 32 x 64 and in 32 x 32; 300 x 1024
+// 71, 40, 41 and 33 (chosen, as 16 x 64). Tiles of 128 x 128, 88 x 128 and 64 x 192 and packed multiply-adds on pairs of rows
+// and columns were no faster at any of these sizes (514 x 5632: 161 us in 64 x 128, packed 174).
 struct F32Choice { int bm, bn; float few, full, two, three, four, more; };
-static const F32Choice kF32Tiles[] = {{64, 128, 72.f, 72.f, 126.f, 162.f, 226.f, 38.f}, {64, 64, 40.f, 41.f, 70.f, 106.f, 115.f, 26.f},
-                                      {32, 64, 24.f, 26.f, 43.f, 58.f, 81.f, 12.f}, {32, 32, 16.6f, 18.f, 26.f, 37.5f, 57.f, 8.4f},
-                                      {16, 64, 17.7f, 20.5f, 27.7f, 37.6f, 55.f, 8.4f}, {16, 32, 13.f, 16.3f, 30.f, 41.f, 48.5f, 11.f},
-                                      {8, 64, 13.9f, 20.f, 30.f, 33.f, 52.f, 9.5f}, {4, 64, 11.4f, 15.f, 24.f, 26.f, 34.6f, 9.f}};
+static const F32Choice kF32Tiles[] = {{64, 128, 71.f, 72.f, 125.f, 162.f, 215.f, 53.f}, {64, 64, 39.5f, 40.5f, 63.f, 86.f, 114.f, 27.3f},
+                                      {32, 64, 24.3f, 25.5f, 41.f, 51.5f, 66.f, 14.7f}, {32, 32, 16.9f, 17.5f, 25.f, 33.f, 41.f, 9.5f},
+                                      {16, 64, 18.f, 19.5f, 26.f, 33.f, 42.5f, 9.8f}, {16, 32, 13.f, 14.f, 23.5f, 31.f, 41.f, 9.6f},
+                                      {8, 64, 13.9f, 14.7f, 24.5f, 33.f, 44.f, 10.3f}, {4, 64, 11.4f, 13.f, 19.f, 26.f, 34.f, 8.f}};
 
 static float f32_cost(const F32Choice& t, int M, int N, int sms) {
     const long long units = (long long)((M + t.bm - 1) / t.bm) * ((N + t.bn - 1) / t.bn), rounds = (units + sms - 1) / sms;
@@ -149,12 +170,7 @@ static float f32_cost(const F32Choice& t, int M, int N, int sms) {
 }
 // the tile of the least estimated time among those whose grid is not too tall, or -1
 static int f32_tile(int M, int N) {
-    static int sms = 0;
-    if (!sms) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
-    }
+    const int sms = f32_sms();
     int best = -1;
     float best_cost = 0.0f;
     for (int i = 0; i < (int)(sizeof(kF32Tiles) / sizeof(kF32Tiles[0])); i++) {
