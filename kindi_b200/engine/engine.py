@@ -50,7 +50,9 @@ class Engine:
         """``model_dir``: a folder with config.json and safetensors files; or give ``spec`` and ``tensors``
         directly. ``ctx``: the most tokens all live sequences hold together (rounded up per sequence to the cache
         page); it sizes the cache, like the reference's ``ctx`` (``kindi/nanbeige.py:245``). ``prompt_graph_tokens``:
-        prompt steps of up to this many tokens are recorded too, padded to a multiple of 64 rows (0: never)."""
+        prompt steps of up to this many tokens are recorded too, padded to a multiple of 64 rows (0: never); from 512 on,
+        longer ones as well, as long as the host would take longer to issue them than the GPU to run them
+        (``long_prompt_tokens``)."""
         if dtype not in _DTYPES:
             raise EngineError("dtype must be 'bfloat16' or 'float32', not %r" % (dtype,))
         if not torch.cuda.is_available():
@@ -92,6 +94,46 @@ class Engine:
         self._graphs: Dict[tuple, "_StepGraph"] = {}
         self.graph_replays = 0
         self._graph_warm = set()
+        self.long_prompt_tokens = self._long_prompt_tokens() if self.cuda_graphs else 0
+        self._long_pool = None                         # the memory that recordings of long prompts share
+        self.long_graphs_kept = 24
+
+    # Recordings of longer prompts. A step that is issued launch by launch costs the host about 150 us a layer (a prompt of
+    # 600 tokens through four layers of width 1024: 725 us, 292 recorded; of 1300: 750, 415; two expert layers of 2048 at
+    # 2048 tokens 648, 594); where the GPU needs longer than that (3B-shaped layers from 700 tokens on: 836, 859 at 1300)
+    # nothing is gained. HOST_US_PER_LAYER and the rates (multiplications a microsecond at the products' usual speed) draw
+    # that line; the recordings share one pool of memory, for as many rows as fit what the memory plan leaves over.
+    HOST_US_PER_LAYER = 150.0
+    FLOP_PER_US = {torch.bfloat16: 1.0e9, torch.float32: 4.0e7}
+    LONG_PROMPT_MOST = 4096
+    LONG_LOGITS_BYTES = 64 << 20                       # (each recording keeps its own logits)
+
+    def record_stream(self) -> torch.cuda.Stream:
+        """the side stream that steps are recorded on"""
+        if getattr(self, "_record_stream", None) is None:
+            self._record_stream = torch.cuda.Stream(self.device)
+        return self._record_stream
+
+    def _long_prompt_tokens(self) -> int:
+        """the most tokens of a prompt step that is recorded beyond ``prompt_graph_tokens`` (0: none)"""
+        if self.prompt_graph_tokens < 512:
+            return 0
+        el = 4 if self.dtype == torch.float32 else 2
+        us_per_row = 0.0
+        for e in self.spec.schedule:
+            block = self.model.blocks[e.layer]
+            us_per_row += 2.0 * block.bytes_read() / el / self.FLOP_PER_US[self.dtype] + block.recorded_us_per_row()
+        rows = self.HOST_US_PER_LAYER * len(self.spec.schedule) / max(us_per_row, 1e-9)
+        rows = int(min(rows, self.LONG_PROMPT_MOST, self.max_step_tokens, self.ctx)) // 64 * 64
+        spare = self.plan["free"] - self.plan["total"]
+        while rows > self.prompt_graph_tokens and 2 * rows * self.plan["per_row"] + self.long_graphs_kept_bytes() > spare:
+            rows -= 64
+        return rows if rows > self.prompt_graph_tokens else 0
+
+    @classmethod
+    def long_graphs_kept_bytes(cls) -> int:
+        """what the kept recordings' logits may take together"""
+        return 24 * cls.LONG_LOGITS_BYTES
 
     def _plan_memory(self, spec: ModelSpec, tensors) -> Dict[str, int]:
         """what the engine will hold on the device, counted before anything is allocated: the weights (twice the
@@ -116,7 +158,7 @@ class Engine:
         per_row = 3 * spec.width * 4 + 2 * widest * max(el, 2)
         work = (rows + self.prompt_graphs_kept * self.prompt_graph_tokens) * per_row \
             + self.max_batch * spec.vocab_size * 4 * 2
-        plan = {"weights": weights, "cache": cache, "work": work, "total": weights + cache + work}
+        plan = {"weights": weights, "cache": cache, "work": work, "total": weights + cache + work, "per_row": per_row}
         free, total = torch.cuda.mem_get_info(self.device)
         plan["free"] = int(free)
         gib = 2.0 ** 30
@@ -180,7 +222,11 @@ class Engine:
                     key = ("decode", len(entries))
             elif n_tok <= self.prompt_graph_tokens and not tokens_from_previous:
                 key = ("prompt", (n_tok + 63) // 64 * 64, len(entries), sum(len(e.want) for e in entries))
-        ps = pack(entries, before, pad_rows_to=key[1] if key and key[0] == "prompt" else 0)
+            elif self.prompt_graph_tokens < n_tok <= self.long_prompt_tokens and not tokens_from_previous:
+                wanted = sum(len(e.want) for e in entries)
+                if wanted * self.spec.vocab_size * 4 <= self.LONG_LOGITS_BYTES:
+                    key = ("long prompt", (n_tok + 63) // 64 * 64, len(entries), wanted)
+        ps = pack(entries, before, pad_rows_to=key[1] if key and key[0] != "decode" else 0)
         reserved = []
         try:
             for e, new_len in zip(entries, ps.h_kv_len):
@@ -194,11 +240,21 @@ class Engine:
         if key is not None:
             graph = self._graphs.get(key)
             if graph is None and key in self._graph_warm:
-                if key[0] == "prompt":
-                    kept = [k for k in self._graphs if k[0] == "prompt"]
-                    if len(kept) >= self.prompt_graphs_kept:
+                pool = None
+                if key[0] != "decode":
+                    kept = [k for k in self._graphs if k[0] == key[0]]
+                    if len(kept) >= (self.prompt_graphs_kept if key[0] == "prompt" else self.long_graphs_kept):
                         del self._graphs[kept[0]]              # the oldest recorded prompt shape makes room
-                graph = self._graphs[key] = _StepGraph(self, ps)
+                        if key[0] == "long prompt":            # (and has to come twice again: a recording costs some steps' gain)
+                            self._graph_warm.discard(kept[0])
+                            if len(kept) == 1:
+                                self._long_pool = None         # (a pool lives as long as its recordings)
+                        torch.cuda.empty_cache()               # its memory goes back
+                if key[0] == "long prompt":
+                    if self._long_pool is None:
+                        self._long_pool = torch.cuda.graph_pool_handle()
+                    pool = self._long_pool
+                graph = self._graphs[key] = _StepGraph(self, ps, pool)
             self._graph_warm.add(key)
             if graph is None and ps.T != n_tok:
                 ps = pack(entries, before)                     # not recorded (yet): run it without the padding rows
@@ -395,7 +451,9 @@ class _StepGraph:
     """the recorded launch sequence of one step shape (a decode step of B sequences, or a prompt step of so many rows,
     sequences and wanted rows), over fixed device buffers"""
 
-    def __init__(self, engine: Engine, ps: PackedStep):
+    def __init__(self, engine: Engine, ps: PackedStep, pool=None):
+        """``pool``: memory to share with other recordings (they are replayed on one stream, and a step's logits hold until
+        the engine's next step only)"""
         self.engine = engine
         n = ps.meta.size
         self.pin = torch.empty(n, dtype=torch.int32, pin_memory=True)
@@ -408,18 +466,27 @@ class _StepGraph:
         rows = self.meta[a:a + m]
         self.graph = torch.cuda.CUDAGraph()
         # Nothing but this library's launches may happen while the stream records: a garbage collection that frees
-        # pinned buffers of an earlier engine would query events, which invalidates a recording in the strict mode.
+        # pinned buffers of an earlier engine would query events, which invalidates a recording in the strict mode. (torch's
+        # own context manager collects garbage and gives back all cached memory before every recording, 70 ms each; with the
+        # collector off that is only needed where the recording's memory might not be there otherwise.)
         import gc
-        gc.collect()
-        torch.cuda.synchronize()
+        free, _ = torch.cuda.mem_get_info(engine.device)
+        if free < (2 << 30) + 4 * ps.T * engine.plan["per_row"]:
+            gc.collect()
+            torch.cuda.empty_cache()
         n0 = K.launch_count()
         was_on = gc.isenabled()
         gc.disable()
         try:
-            with torch.cuda.graph(self.graph, capture_error_mode="relaxed"):
-                self.logits = engine.model.forward(ctx, rows)
-                # the greedy pick rides along (a step that wants no row has nothing to pick)
-                self.picked = engine.pick(self.logits, _GREEDY) if self.logits is not None else None
+            torch.cuda.synchronize()
+            with torch.cuda.stream(engine.record_stream()):
+                self.graph.capture_begin(*(() if pool is None else (pool,)), capture_error_mode="relaxed")
+                try:
+                    self.logits = engine.model.forward(ctx, rows)
+                    # the greedy pick rides along (a step that wants no row has nothing to pick)
+                    self.picked = engine.pick(self.logits, _GREEDY) if self.logits is not None else None
+                finally:
+                    self.graph.capture_end()
         finally:
             if was_on:
                 gc.enable()

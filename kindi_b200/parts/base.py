@@ -187,6 +187,11 @@ class Part:
         """bytes of weights one step reads (for the roofline account)"""
         return 0
 
+    def recorded_us_per_row(self) -> float:
+        """what a recorded long prompt costs more a row than the same step issued launch by launch (microseconds): a part whose
+        best form needs the step's host-side numbers, which a recording does not have"""
+        return 0.0
+
 
 class Norm(Part):
     category = "norm"

@@ -116,6 +116,9 @@ class PreNormBlock(Block):
     def bytes_read(self) -> int:
         return sum(p.bytes_read() for p in self._parts())
 
+    def recorded_us_per_row(self) -> float:
+        return sum(p.recorded_us_per_row() for p in self._parts())
+
 
 class SandwichBlock(PreNormBlock):
     """a norm before AND after every sub-layer: ``x += norm1b(mixer(norm1(x)))``, then ``x += norm2b(feed_forward(norm2(x)))``.

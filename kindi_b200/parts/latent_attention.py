@@ -170,5 +170,9 @@ class LatentAttention(Mixer):
     def bytes_read(self) -> int:
         return sum(w.numel() * w.element_size() for w in (self.w_down, self.w_uq, self.w_uk_t, self.w_uv, self.w_o))
 
+    def recorded_us_per_row(self) -> float:
+        # (the form over expanded keys and values is out of reach: the per-head products instead, see fast.latent_full_pays)
+        return self.H * self.kr * (self.d + self.dv) * 2e-8 if self.w_kv is not None else 0.0
+
 
 register_part("mixer", "latent_attention", LatentAttention)

@@ -85,5 +85,8 @@ class ParallelMixers(Mixer):
     def bytes_read(self) -> int:
         return sum(m.bytes_read() for m in self.mixers)
 
+    def recorded_us_per_row(self) -> float:
+        return sum(m.recorded_us_per_row() for m in self.mixers)
+
 
 register_part("mixer", "parallel", ParallelMixers)

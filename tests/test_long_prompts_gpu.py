@@ -1,0 +1,64 @@
+"""Recorded prompt steps of more than 512 tokens: padded rows, several sequences, cached positions in front, shapes that share
+one pool of memory and take turns, and a shape that was dropped. Compared with the plain implementation."""
+import random
+
+import numpy as np
+import pytest
+
+import plain_model as P
+import tiny
+
+pytestmark = pytest.mark.gpu
+TOL = {"bfloat16": 1.5e-2, "float32": 2e-5}
+
+
+@pytest.mark.parametrize("dtype", ["bfloat16", "float32"])
+def test_long_prompts_are_recorded(tmp_path, dtype):
+    from kindi_b200.engine.batch import StepEntry
+    from kindi_b200.engine.engine import Engine
+    folder = tiny.make_model(tmp_path, "D", dtype)
+    vocab = tiny.TINY["D"][0]["vocab_size"]
+    m = P.load_model(folder)
+    eng = Engine(folder, ctx=8192, dtype=dtype, max_batch=3)
+    assert eng.long_prompt_tokens >= 1024, eng.long_prompt_tokens
+    rng = random.Random(9)
+    toks = lambda n: [rng.randrange(vocab) for _ in range(n)]                       # noqa: E731
+    # (lengths of a step's sequences): shapes come twice and more, in turns
+    for lens in ([520], [575], [300, 290, 17], [560], [280, 300, 27], [700], [1], [703], [301, 1, 300], [520]):
+        seqs = [toks(n) for n in lens]
+        slots = [eng.alloc() for _ in seqs]
+        got = eng.step([StepEntry(s, tuple(t), (len(t) - 1,)) for s, t in zip(slots, seqs)]).cpu().numpy()
+        more = [toks(400) for _ in seqs]                                             # a further turn on top of them
+        got2 = eng.step([StepEntry(s, tuple(t), (0, len(t) - 1)) for s, t in zip(slots, more)]).cpu().numpy()
+        eng.check_status()
+        for i, (s, t, u) in enumerate(zip(slots, seqs, more)):
+            want = P.forward(m, t + u).numpy()
+            assert tiny.rel_err(got[i], want[len(t) - 1]) <= TOL[dtype], (lens, i)
+            assert tiny.rel_err(got2[2 * i:2 * i + 2], want[[len(t), len(t) + 399]]) <= TOL[dtype], (lens, i)
+            eng.free(s)
+    kinds = {k[:3] for k in eng._graphs if k[0] == "long prompt"}
+    assert ("long prompt", 576, 1) in kinds and ("long prompt", 640, 3) in kinds and ("long prompt", 704, 1) in kinds, kinds
+    eng.cache.check()
+
+
+def test_long_prompt_shapes_are_kept_up_to_a_limit(tmp_path):
+    from kindi_b200.engine.batch import StepEntry
+    from kindi_b200.engine.engine import Engine
+    folder = tiny.make_model(tmp_path, "D", "bfloat16")
+    vocab = tiny.TINY["D"][0]["vocab_size"]
+    m = P.load_model(folder)
+    eng = Engine(folder, ctx=4096, dtype="bfloat16", max_batch=1)
+    eng.long_graphs_kept = 1
+    off = Engine(folder, ctx=4096, dtype="bfloat16", max_batch=1, prompt_graph_tokens=128)
+    assert off.long_prompt_tokens == 0                    # (a caller's own limit below the default stays the limit)
+    rng = random.Random(4)
+    for n in (550, 560, 620, 630, 540, 570, 565):
+        t = [rng.randrange(vocab) for _ in range(n)]
+        s = eng.alloc()
+        got = eng.step([StepEntry(s, tuple(t), (n - 1,))])[0].cpu().numpy()
+        eng.check_status()
+        eng.free(s)
+        assert tiny.rel_err(got, P.forward(m, t).numpy()[-1]) <= TOL["bfloat16"], n
+        assert sum(1 for k in eng._graphs if k[0] == "long prompt") <= 1
+    # the first shape was dropped for the second and recorded again only once it had come twice
+    assert [k[1] for k in eng._graphs if k[0] == "long prompt"] == [576] and np.isfinite(got).all()
