@@ -1,0 +1,299 @@
+// Products of a few rows with the experts they chose (up to 8 rows, 64 picks), straight from the router's picks.
+//
+// A decode step of eight rows that each choose 4 of 32 experts touches about 20 of them with one or two rows each: the step
+// streams their matrices and computes next to nothing. The grouped products (moe_tc.cu) need the picks sorted into tiles
+// (k_moe_plan) and the rows gathered (k_moe_gather) first, two dependent launches of about 3 us, and deal an expert's matrix
+// out in tiles of 128 rows x 256 columns. Here every block makes the list of the experts that were chosen itself, the
+// outputs of all of them stand in one line, and block c takes the c-th even stretch of it over the whole of K, as in
+// gemv.cu: warps share K, weights come through rings of copies (128 to 160 KB in flight a block), sums meet in shared memory
+// in the warps' order.
+//   - up: all rows of the step are multiplied with every row of weights (they are the narrow side of the tensor product: eight
+//     cost what one costs); the epilogue keeps the rows that chose the expert and applies the activation;
+//   - down: a tile lies within one expert, and the narrow side holds the picks' own rows of h, which come with the weights;
+//     out = the weighted product in plane k of the pick's row.
+// A row's bits do not depend on which other rows chose an expert.
+// Measured in a recorded step of eight rows, 4 of 32 experts of 1024, width 2048 (about 21 experts touched, 13.4 us a product at
+// the copy rate): plan, gather, up and down 3 + 3 + 22 + 23 us -> up and down 20 + 20.5. Sixteen warps with two copies each:
+// 20.3 + 20.5; eight with four 20.5 + 23 (a warp waits for its own copies to be taken in, and does nothing else meanwhile).
+#include "mma_sync.cuh"
+#include "sm100.cuh"
+
+#define MG_ROWS 8                       // rows of a step
+#define MG_PICKS 64
+#define MG_EXPERTS 256
+#define MG_TILES 128                    // tiles a block can have
+
+struct MgArgs {
+    const bf16* A;                      // up: [T][lda] rows; down: [T top][lda] h
+    const bf16* W;                      // [experts][R][K]
+    const int* idx;                     // [T][top]
+    const float* wts;                   // down: [T][top]
+    int T, top, n_exp, R, K, lda;
+    void* out;                          // up: bf16 [T top][R]; down: float [top][T][R]
+    int act, act_off, red_off, ks;      // ks: warps that share K
+    int* status;
+};
+
+// WARPS: 16 with two copies of a tile in flight each, or 8 with three (rows that leave no room for 16); PASS: tiles of 32 outputs
+// a warp brings to an epilogue
+template <bool UP, int WARPS, int D>
+__global__ void __launch_bounds__(32 * WARPS, 1) k_moe_gemv(const MgArgs a) {
+    constexpr int MG_WARPS = WARPS, MG_THREADS = 32 * WARPS, MG_PASS = 32 / WARPS;
+    extern __shared__ __align__(128) uint8_t mg_smem[];
+    __shared__ __align__(8) uint64_t s_bar;
+    __shared__ unsigned s_mask[MG_EXPERTS / 32];
+    __shared__ int s_list[MG_PICKS];                                 // the chosen experts, in order
+    __shared__ int s_idx[MG_PICKS], s_tile[MG_TILES + 1];            // the picks; where the block's tiles begin
+    __shared__ signed char s_pick[MG_PICKS][MG_ROWS];                // which pick of a row chose the expert (-1: none)
+    kb_pdl_launch_now();
+    constexpr int G = 4, TO = 32, STAGE = (G + (UP ? 0 : 1)) * 1024, TP = MG_ROWS + 1;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, q = lane & 3;
+    // warp (rs, ks): every rs-th tile over the ks-th stretch of K (so that a warp has four blocks of K a tile where K is short)
+    const int KS = a.ks, RS = MG_WARPS / KS, ks = warp % KS, rs = warp / KS;
+    const int n_kb = (a.K + 63) >> 6, k0 = ks * n_kb / KS, k1 = (ks + 1) * n_kb / KS;
+    const int pitch = ((a.K * 2 + 127) & ~127) + 16;
+    uint8_t* s_act = mg_smem + a.act_off;
+    float* s_red = (float*)(mg_smem + a.red_off);
+    float* red = s_red + (size_t)warp * MG_PASS * TO * TP;           // [rs][ks][tile of the pass][output][row]
+    const uint8_t* ring = mg_smem + warp * (D * STAGE);
+    const uint32_t ring_u = smem_u32(ring), bar = smem_u32(&s_bar);
+    if (tid < MG_EXPERTS / 32) s_mask[tid] = 0;
+    if (tid == 0) {
+        mbar_init(bar, 1);
+        mbar_fence_init();
+    }
+    __syncthreads();
+    kb_pdl_wait();
+    if (UP) {
+        // the rows into shared memory (zeros from K to the end of its last block)
+        if (tid == 0) mbar_expect_tx(bar, a.T * a.K * 2);
+        __syncwarp();
+        if (tid < a.T) {
+            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                         ::"r"(smem_u32(s_act + tid * pitch)), "l"(a.A + (size_t)tid * a.lda), "r"(a.K * 2), "r"(bar) : "memory");
+        }
+        for (int t = warp; t < a.T; t += MG_WARPS)
+            for (int z = a.K * 2 + lane * 16; z < n_kb * 128; z += 512) *(uint4*)(s_act + t * pitch + z) = make_uint4(0, 0, 0, 0);
+    }
+    const int n_pick = a.T * a.top;
+    int e = -1;
+    if (tid < n_pick) {
+        e = a.idx[tid];
+        s_idx[tid] = e;
+        if (e >= 0 && e < a.n_exp) atomicOr(&s_mask[e >> 5], 1u << (e & 31));
+    }
+    __syncthreads();
+    int n_list = 0;
+#pragma unroll
+    for (int w = 0; w < MG_EXPERTS / 32; w++) n_list += __popc(s_mask[w]);
+    if (tid < MG_EXPERTS && ((s_mask[tid >> 5] >> (tid & 31)) & 1u)) {
+        int r = __popc(s_mask[tid >> 5] & ((1u << (tid & 31)) - 1u));
+        for (int w = 0; w < (tid >> 5); w++) r += __popc(s_mask[w]);
+        s_list[r] = tid;
+    }
+    __syncthreads();
+    for (int i = tid; i < n_list * MG_ROWS; i += MG_THREADS) {
+        const int t = i % MG_ROWS, ex = s_list[i / MG_ROWS];
+        int k = -1;
+        if (t < a.T)
+            for (int j = 0; j < a.top; j++)
+                if (s_idx[t * a.top + j] == ex) k = j;
+        s_pick[i / MG_ROWS][t] = (signed char)k;
+    }
+    const int n_out = n_list * a.R;
+    const int o0 = (int)(blockIdx.x * (unsigned long long)n_out / gridDim.x), o1 = (int)((blockIdx.x + 1) * (unsigned long long)n_out / gridDim.x);
+    // tiles: up to 32 outputs of one expert
+    int tiles = 0;
+    for (int o = o0, end = (o0 / a.R + 1) * a.R; o < o1;) {
+        if (tid == 0) s_tile[tiles] = o;
+        o = min(o1, min(o + TO, end));
+        if (o == end) end += a.R;
+        tiles++;
+    }
+    if (tid == 0) s_tile[tiles] = o1;
+    __syncthreads();
+    const int mine = tiles > rs ? (tiles - rs + RS - 1) / RS : 0, total = mine * (k1 - k0);
+
+    const int cr = lane >> 3, pc = lane & 7;
+    const uint32_t cd0 = ring_u + cr * 128 + ((pc ^ cr) << 4), cd1 = ring_u + cr * 128 + ((pc ^ (cr + 4)) << 4);
+    const bf16 *src = a.W, *ha[2] = {a.A, a.A};
+    uint32_t on = 0, on_a = 0;
+    int l_t = rs, l_k = k0;
+    auto rows_of_tile = [&]() {
+        if (l_t >= tiles) return;
+        const int o = s_tile[l_t], s = o / a.R, rows = s_tile[l_t + 1] - o;
+        src = a.W + ((size_t)s_list[s] * a.R + (o - s * a.R) + cr) * a.K + pc * 8;
+        on = 0;
+#pragma unroll
+        for (int j = 0; j < 8; j++) on |= cr + 4 * j < rows ? 1u << j : 0u;
+        if (!UP) {
+            on_a = 0;
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const int k = s_pick[s][cr + 4 * h];
+                if (k >= 0) {
+                    on_a |= 1u << h;
+                    ha[h] = a.A + (size_t)((cr + 4 * h) * a.top + k) * a.lda + pc * 8;
+                }
+            }
+        }
+    };
+    auto copy16 = [](uint32_t dst, const void* p, int bytes, uint32_t yes) {
+        asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %3, 0;\n @p cp.async.cg.shared.global [%0], [%1], 16, %2;\n}"
+                     ::"r"(dst), "l"(p), "r"(bytes), "r"(yes) : "memory");
+    };
+    auto load = [&](int slot) {
+        const bool ok = l_k * 64 + pc * 8 < a.K;
+        const int bytes = ok ? 16 : 0;
+        const bf16* p = ok ? src + l_k * 64 : a.W;
+        const size_t step = ok ? (size_t)4 * a.K : 0;
+        const uint32_t d = slot * STAGE;
+#pragma unroll
+        for (int j = 0; j < 8; j++) copy16((j & 1 ? cd1 : cd0) + d + j * 512, p + j * step, bytes, on & (1u << j));
+        if (!UP) {
+            // (rows that did not choose the expert: what is there gives sums nobody reads)
+            copy16(cd0 + d + G * 1024, ok ? ha[0] + l_k * 64 : a.A, bytes, on_a & 1u);
+            copy16(cd1 + d + G * 1024 + 512, ok ? ha[1] + l_k * 64 : a.A, bytes, on_a & 2u);
+        }
+        if (++l_k == k1) {
+            l_k = k0;
+            l_t += RS;
+            rows_of_tile();
+        }
+    };
+    rows_of_tile();
+#pragma unroll
+    for (int d = 0; d < D; d++) {
+        if (d < total) load(d);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    bool good = true;
+    if (UP) good = mbar_wait(bar, 0, a.status);
+    if (__syncthreads_or(!good)) {
+        cp_async_wait_all();
+        mbar_wait_ns(bar, 0, a.status, 10000000ull);
+        return;
+    }
+    const uint32_t rd0 = g * 128 + (((2 * q) ^ g) << 4), rd1 = g * 128 + (((2 * q + 1) ^ g) << 4);
+    const uint8_t* arow = s_act + min(g, a.T - 1) * pitch + q * 32;
+    int slot = 0, s_no = 0;
+    for (int p0 = 0; p0 < tiles; p0 += MG_PASS * RS) {
+        for (int t = 0; t < MG_PASS && p0 + t * RS + rs < tiles; t++) {
+            float acc[2][4];
+#pragma unroll
+            for (int m = 0; m < 2; m++)
+#pragma unroll
+                for (int c = 0; c < 4; c++) acc[m][c] = 0.0f;
+            for (int kb = k0; kb < k1; kb++, s_no++) {
+                asm volatile("cp.async.wait_group %0;" ::"n"(D - 1) : "memory");
+                __syncwarp();
+                const uint8_t* st = ring + slot * STAGE;
+                uint32_t wv[G][8], bx[8];
+#pragma unroll
+                for (int i = 0; i < G; i++) {
+                    *(uint4*)&wv[i][0] = *(const uint4*)(st + i * 1024 + rd0);
+                    *(uint4*)&wv[i][4] = *(const uint4*)(st + i * 1024 + rd1);
+                }
+                *(uint4*)&bx[0] = UP ? *(const uint4*)(arow + kb * 128) : *(const uint4*)(st + G * 1024 + rd0);
+                *(uint4*)&bx[4] = UP ? *(const uint4*)(arow + kb * 128 + 16) : *(const uint4*)(st + G * 1024 + rd1);
+                __syncwarp();
+                if (s_no + D < total) load(slot);
+                asm volatile("cp.async.commit_group;" ::: "memory");
+                if (++slot == D) slot = 0;
+#pragma unroll
+                for (int j = 0; j < 4; j++)
+#pragma unroll
+                    for (int m = 0; m < 2; m++) {
+                        const uint32_t fa[4] = {wv[2 * m][2 * j], wv[2 * m + 1][2 * j], wv[2 * m][2 * j + 1], wv[2 * m + 1][2 * j + 1]};
+                        mma_bf16(acc[m], fa, bx[2 * j], bx[2 * j + 1]);
+                    }
+            }
+#pragma unroll
+            for (int m = 0; m < 2; m++)
+#pragma unroll
+                for (int c = 0; c < 4; c++)
+                    red[(t * TO + (m * 2 + (c >> 1)) * 8 + g) * TP + q * 2 + (c & 1)] = acc[m][c];
+        }
+        __syncthreads();
+        // the warps' sums in their order: a warp a row of the step, lanes over the pass's outputs
+        const int row = warp % MG_ROWS;
+        for (int t = warp / MG_ROWS; t < MG_PASS * RS && p0 + t < tiles; t += MG_WARPS / MG_ROWS) {
+            const int o = s_tile[p0 + t], rows = s_tile[p0 + t + 1] - o, s = o / a.R, f = o - s * a.R + lane;
+            const int k = s_pick[s][row];
+            if (k >= 0 && lane < rows) {
+                float v = 0.0f;
+                const float* r = s_red + ((size_t)(t % RS) * KS * MG_PASS * TO + (t / RS) * TO + lane) * TP + row;
+                for (int w = 0; w < KS; w++) v += r[(size_t)w * MG_PASS * TO * TP];
+                const int pick = row * a.top + k;
+                if (UP) ((bf16*)a.out)[(size_t)pick * a.R + f] = __float2bfloat16_rn(kb_act(v, a.act));
+                else ((float*)a.out)[((size_t)k * a.T + row) * a.R + f] = a.wts[pick] * v;
+            }
+        }
+        __syncthreads();
+    }
+    cp_async_wait_all();
+}
+
+// warps of a block and its shared memory (0: no room)
+static int mg_plan(int T, int K, int up, MgArgs* a, int* warps) {
+    const int pitch = ((K * 2 + 127) & ~127) + 16, act = up ? T * pitch : 0, red = 32 * 32 * (MG_ROWS + 1) * 4;
+    for (int w = 16; w >= 8; w /= 2) {
+        const int ring = w * (w == 16 ? 2 : 3) * (up ? 4096 : 5120);
+        if (ring + act + red > 224 * 1024) continue;
+        a->act_off = ring;
+        a->red_off = ring + act;
+        *warps = w;
+        return ring + act + red;
+    }
+    return 0;
+}
+
+static int mg_blocks() {
+    int dev = 0, n = 0;
+    cudaGetDevice(&dev);
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
+    return n;
+}
+// whether a block's tiles fit its list: its stretch in tiles, and one more at every expert it touches
+static int mg_fits(int picks, int n_exp, int R) {
+    const long long n = picks < n_exp ? picks : n_exp, part = n * R / mg_blocks() + 1;
+    return part / 32 + part / R + 4 <= MG_TILES;
+}
+
+// 1 when kb_moe_gemv takes the step
+extern "C" int kb_moe_gemv_takes(int T, int top, int n_exp, int width, int F) {
+    MgArgs a;
+    int d;
+    return T >= 1 && T <= MG_ROWS && top >= 1 && T * top <= MG_PICKS && n_exp <= MG_EXPERTS && width >= 64 && F >= 64 &&
+           width % 16 == 0 && F % 16 == 0 && mg_fits(T * top, n_exp, F) && mg_fits(T * top, n_exp, width) && mg_plan(T, width, 1, &a, &d) && mg_plan(T, F, 0, &a, &d);
+}
+
+template <bool UP, int WARPS, int D>
+static int mg_launch(const MgArgs& a, int smem, cudaStream_t st) {
+    auto kern = k_moe_gemv<UP, WARPS, D>;
+    static char once_tag;
+    if (kb_first_use(&once_tag)) {
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 225 * 1024);
+        if (e != cudaSuccess) return (int)e;
+    }
+    kb_launch(kern, mg_blocks(), 32 * WARPS, smem, st, a);
+    return (int)cudaGetLastError();
+}
+
+// up: out bf16 [T top][R] = act(W[idx] A_t) for every pick; down (up == 0): out float [top][T][R] = wts W[idx] A_pick. W is
+// [n_exp][R][K]. Picks that name no expert are left out.
+extern "C" int kb_moe_gemv(const void* A, int lda, const void* W, const int* idx, const float* wts, int T, int top, int n_exp, int R,
+                           int K, void* out, int up, int act, int* status, cudaStream_t st) {
+    if (T < 1 || T > MG_ROWS || top < 1 || T * top > MG_PICKS || n_exp < 1 || n_exp > MG_EXPERTS || R < 1 || K < 16 || (K & 15) || (lda & 7) ||
+        ((uintptr_t)A & 15) || ((uintptr_t)W & 15) || (!up && !wts) || !mg_fits(T * top, n_exp, R) || (long long)T * top * R > 0x7fffffffLL)
+        return (int)cudaErrorInvalidValue;
+    MgArgs a = {};
+    a.A = (const bf16*)A; a.W = (const bf16*)W; a.idx = idx; a.wts = wts;
+    a.T = T; a.top = top; a.n_exp = n_exp; a.R = R; a.K = K; a.lda = lda; a.out = out; a.act = act; a.status = status;
+    int warps = 0;
+    const int smem = mg_plan(T, K, up, &a, &warps), n_kb = (K + 63) / 64;
+    if (!smem) return (int)cudaErrorInvalidValue;
+    a.ks = n_kb >= 4 * warps ? warps : n_kb >= 32 ? 8 : n_kb >= 16 ? 4 : n_kb >= 8 ? 2 : 1;
+    if (up) return warps == 16 ? mg_launch<true, 16, 2>(a, smem, st) : mg_launch<true, 8, 3>(a, smem, st);
+    return warps == 16 ? mg_launch<false, 16, 2>(a, smem, st) : mg_launch<false, 8, 3>(a, smem, st);
+}

@@ -153,6 +153,9 @@ def _prefill_product(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, status
 # up to here a product may go through the kernel whose blocks finish their outputs (16 rows: its down product of 2560 x 10496
 # takes 15.9 us, the tensor-memory form 11.6: every block reads all activation rows)
 GEMV_ROWS = 8
+# finished 32-bit rows of so few outputs go there too: the tensor-memory form would give each tile of 128 outputs the whole of
+# K on one SM (a router of 32 experts over 2048, eight rows: 11.2 us, 3.6 here); the head's many tiles stream at 6.5 TB/s
+GEMV_FEW_OUTPUTS = 32 * 148
 
 
 def gemv_ok(m: int, lda: int, w: torch.Tensor, glu: bool = False, squares: bool = False) -> bool:
@@ -165,7 +168,9 @@ def gemm_rows(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, status: torch
     if not _tc_ok(a, w) or not out.is_contiguous():
         return False
     m, n = a.shape[0], w.shape[0]
-    if m <= SMALL_M:
+    if n <= GEMV_FEW_OUTPUTS and out.dtype == torch.float32 and gemv_ok(m, a.stride(0), w):
+        K.gemv(a, w, out, status)
+    elif m <= SMALL_M:
         K.gemm_tc(a, w, out, swap=True, bn=_swap_bn(m), splits=1, status=status)
     else:
         _prefill_product(a, w, out, status, False)
@@ -458,6 +463,13 @@ def moe_experts(ctx, y, idx, wts, wup, wdown, top, act, gated=False, weight_on="
     E, F, _ = wup.shape
     if not _moe_tc_ok(y, wup, wdown) or (gated and (F // 2) % 8):
         return None
+    if (not gated and wup.data_ptr() % 16 == 0 and wdown.data_ptr() % 16 == 0 and wup.is_contiguous() and wdown.is_contiguous()
+            and K.moe_gemv_takes(T, top, E, width, F)):
+        h = torch.empty((T * top, F), dtype=torch.bfloat16, device=y.device)
+        planes = torch.empty((top, T, width), dtype=torch.float32, device=y.device)
+        K.moe_gemv(y, wup, idx, None, h, ctx.status, up=True, act=act)
+        K.moe_gemv(h, wdown, idx, wts, planes, ctx.status, up=False)
+        return planes
     plan = K.moe_plan(idx, E, K.moe_gemm_tc_tile())
     ys = torch.empty((T * top, width), dtype=torch.bfloat16, device=y.device)
     K.moe_gather(y, ys, plan, top)

@@ -129,6 +129,9 @@ _SIGS = {
     "kb_moe_gemm_tc": [c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_int, c_void_p, c_int, c_longlong, c_int,
                        c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
                        c_void_p, c_void_p, c_int, c_float, c_float],
+    "kb_moe_gemv_takes": [c_int, c_int, c_int, c_int, c_int],
+    "kb_moe_gemv": [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int, c_int,
+                    c_void_p, c_void_p],
     "kb_moe_gather": [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p],
     "kb_moe_gemm": [c_void_p, c_int, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_longlong, c_int, c_int, c_int,
                     c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p],
@@ -229,6 +232,7 @@ class KernelTiming:
     def __getattr__(self, name):                       # stands in for the library while timing is on
         fn = getattr(_lib, name)
         if not name.startswith("kb_") or name in ("kb_set_pdl", "kb_gemm_tc_splits", "kb_rope_table_min_rows", "kb_gemv_blocks", "kb_gemv_takes",
+                                                  "kb_moe_gemv_takes",
                                                   "kb_moe_gemm_tile", "kb_moe_gemm_tc_tile", "kb_scan_run",
                                                   "kb_wkv_run"):
             return fn
@@ -766,6 +770,30 @@ def moe_gemm_tc(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, plan: MoePl
                                  _p(plan.perm), _p(wts), top, GATE_ACT[act] if glu else ACT[act], 1 if up else 0, bn,
                                  _p(status), _stream(), 1 if glu else 0, *_gate_params(act if glu else "", act_params)),
            "moe_gemm_tc")
+
+
+@functools.lru_cache(maxsize=256)
+def moe_gemv_takes(T: int, top: int, n_exp: int, width: int, f: int) -> bool:
+    return bool(load().kb_moe_gemv_takes(T, top, n_exp, width, f))
+
+
+def moe_gemv(a: torch.Tensor, w: torch.Tensor, idx: torch.Tensor, wts: Optional[torch.Tensor], out: torch.Tensor, status: torch.Tensor,
+             *, up: bool, act: str = "none") -> None:
+    """a few rows' products with the experts they chose (``idx`` int32 [T, top]; w [E, N, K] bf16), without a plan. up: a [T,
+    K], out bf16 [T * top, N] = act(w[idx] a_t), row t * top + k for pick k; else a [T * top, K] such rows and out float32
+    planes [top, T, N] = wts * w[idx] a. Picks that name no expert are left out"""
+    _need_cuda(a, w, idx, wts, out)
+    T, top = idx.shape
+    E, N, k = w.shape
+    assert a.dtype == w.dtype == torch.bfloat16 and w.is_contiguous() and a.stride(1) == 1 and out.is_contiguous()
+    assert idx.dtype == torch.int32 and idx.is_contiguous() and a.shape == ((T if up else T * top), k)
+    if up:
+        assert out.dtype == torch.bfloat16 and out.shape == (T * top, N)
+    else:
+        assert out.dtype == torch.float32 and out.shape == (top, T, N)
+        assert wts is not None and wts.dtype == torch.float32 and wts.is_contiguous() and wts.numel() == T * top
+    _check(load().kb_moe_gemv(_p(a), a.stride(0), _p(w), _p(idx), _p(wts), T, top, E, N, k, _p(out), 1 if up else 0, ACT[act],
+                              _p(status), _stream()), "moe_gemv")
 
 
 def gemm_simt(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:

@@ -1,0 +1,66 @@
+"""Products of a few rows with the experts they chose (``moe_gemv.cu``), against the product in 64 bits: one and eight rows,
+experts that several rows chose, stretches that end inside a tile and span experts, K with a partial block and with fewer
+blocks than warps, more experts than picks, one expert, picks that name none."""
+import pytest
+import torch
+
+from kindi_b200.kernels import lib as K
+
+pytestmark = pytest.mark.gpu
+
+
+def _data(T, top, E, width, F, seed=0):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    y = torch.randn(T, width, device="cuda", generator=g).bfloat16()
+    wu = (torch.randn(E, F, width, device="cuda", generator=g) * 0.05).bfloat16()
+    wd = (torch.randn(E, width, F, device="cuda", generator=g) * 0.05).bfloat16()
+    idx = torch.stack([torch.randperm(E, device="cuda", generator=g)[:top] for _ in range(T)]).int()
+    wts = torch.rand(T, top, device="cuda", generator=g)
+    return y, wu, wd, idx, wts
+
+
+@pytest.mark.parametrize("T,top,E,width,F", [(8, 4, 32, 2048, 1024), (1, 4, 16, 1024, 512), (3, 2, 5, 208, 336), (8, 8, 256, 64, 80),
+                                              (5, 1, 1, 1008, 96), (7, 4, 32, 4096, 2048), (2, 3, 7, 96, 4112), (8, 4, 32, 80, 64)])
+@pytest.mark.parametrize("act", ["relu2", "none"])
+def test_experts_of_a_few_rows(T, top, E, width, F, act):
+    y, wu, wd, idx, wts = _data(T, top, E, width, F)
+    assert K.moe_gemv_takes(T, top, E, width, F)
+    st = torch.zeros(1, dtype=torch.int32, device="cuda")
+    h = torch.full((T * top, F), float("nan"), device="cuda", dtype=torch.bfloat16)
+    planes = torch.full((top, T, width), float("nan"), device="cuda")
+    K.moe_gemv(y, wu, idx, None, h, st, up=True, act=act)
+    K.moe_gemv(h, wd, idx, wts, planes, st, up=False)
+    for t in range(T):
+        for k in range(top):
+            e = int(idx[t, k])
+            u = wu[e].double() @ y[t].double()
+            mag = wu[e].double().abs() @ y[t].double().abs()
+            want, slack = (u.clamp(min=0) ** 2, 2.0 * u.abs() * 2e-6 * mag) if act == "relu2" else (u, 2e-6 * mag)
+            got = h[t * top + k].double()
+            assert ((got - want).abs() <= 2.0 ** -8 * want.abs() + slack + 1e-9).all(), (t, k)
+            w = float(wts[t, k])
+            down, dmag = wd[e].double() @ got, wd[e].double().abs() @ got.abs()
+            assert ((planes[k, t].double() - w * down).abs() <= 2e-6 * w * dmag + 1e-9).all(), (t, k)
+    assert int(st) == 0
+
+
+def test_picks_that_name_no_expert_are_left_alone():
+    y, wu, wd, idx, wts = _data(4, 3, 6, 128, 64, 3)
+    idx[1, 0], idx[2, 2], idx[3] = 6, -1, 99
+    st = torch.zeros(1, dtype=torch.int32, device="cuda")
+    h = torch.full((12, 64), 7.0, device="cuda", dtype=torch.bfloat16)
+    planes = torch.full((3, 4, 128), 7.0, device="cuda")
+    K.moe_gemv(y, wu, idx, None, h, st, up=True)
+    K.moe_gemv(h, wd, idx, wts, planes, st, up=False)
+    for t, k in ((1, 0), (2, 2), (3, 0), (3, 1), (3, 2)):
+        assert (h[t * 3 + k] == 7.0).all() and (planes[k, t] == 7.0).all()
+    assert not (planes[0, 0] == 7.0).any()
+
+
+def test_a_row_does_not_depend_on_the_others():
+    y, wu, wd, idx, wts = _data(8, 4, 16, 512, 256, 5)
+    st = torch.zeros(1, dtype=torch.int32, device="cuda")
+    h, one = (torch.empty(n, 256, device="cuda", dtype=torch.bfloat16) for n in (32, 4))
+    K.moe_gemv(y, wu, idx, None, h, st, up=True, act="silu")
+    K.moe_gemv(y[3:4].contiguous(), wu, idx[3:4].contiguous(), None, one, st, up=True, act="silu")
+    assert torch.equal(one, h[12:16])
