@@ -188,8 +188,8 @@ class Part:
         return 0
 
     def recorded_us_per_row(self) -> float:
-        """what a recorded long prompt costs more a row than the same step issued launch by launch (microseconds): a part whose
-        best form needs the step's host-side numbers, which a recording does not have"""
+        """microseconds a row of a recorded long prompt that ``bytes_read`` at the plain products' rate does not tell: slower
+        products, or a part whose best form needs the step's host-side numbers, which a recording does not have"""
         return 0.0
 
 
