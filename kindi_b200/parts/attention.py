@@ -159,7 +159,8 @@ class CausalSelfAttention(Mixer):
                             float(qkn["eps"]), self.nh * self.qk_dim, self.nkv * self.qk_dim)
 
     def takes_scaled_rows(self, ctx: StepContext) -> bool:
-        return L.takes_scaled(ctx, self.wqkv)
+        # (a part derived from this one may read its rows in a way of its own)
+        return type(self).forward is CausalSelfAttention.forward and L.takes_scaled(ctx, self.wqkv)
 
     def forward(self, ctx: StepContext, y: torch.Tensor) -> Branch:
         nh, nkv, hd = self.nh, self.nkv, self.hd

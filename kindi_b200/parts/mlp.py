@@ -49,7 +49,9 @@ class SwiGLU(FeedForward):
         self.wd = weights(n["down"])
 
     def takes_scaled_rows(self, ctx: StepContext) -> bool:
-        return self.group == L.GATE_UP_GROUP and L.takes_scaled(ctx, self.wgu, glu=True)
+        # (a part derived from this one may read its rows in a way of its own)
+        return (type(self).forward is SwiGLU.forward and self.group == L.GATE_UP_GROUP
+                and L.takes_scaled(ctx, self.wgu, glu=True))
 
     def forward(self, ctx: StepContext, y: torch.Tensor) -> Branch:
         h = L.gate_up_swiglu(ctx, y, self.wgu, self.group, self.f, self.dtype, self.act)

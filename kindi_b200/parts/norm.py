@@ -64,6 +64,8 @@ class RMSNorm(Norm):
     def add_norm_scaled(self, ctx: StepContext, x, pending: Optional[Branch]) -> Optional[ScaledRows]:
         if not isinstance(pending, LazyBranch) or pending.bias is not None or pending.norm is not None:
             return None
+        if type(self).add_norm is not RMSNorm.add_norm:
+            return None                     # (a part derived from this one that norms in a way of its own)
         scale = pending.scale
         if scale is not None and scale.dtype != self.weight.dtype:
             scale = scale.to(self.weight.dtype)
