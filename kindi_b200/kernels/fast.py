@@ -126,6 +126,29 @@ def _prefill_split(m: int, n: int, k: int):
 
 
 _PAIR_SCRATCH = {}         # device -> (partial tiles, flags): scratch of tiles that two pairs of SMs finish together
+_PAIR_RETIRED = []         # scratch that a larger one has taken the place of: a recorded step may still use it
+
+
+def _recording(t: torch.Tensor) -> bool:
+    return t.is_cuda and torch.cuda.is_current_stream_capturing()
+
+
+def _pair_scratch(device, tiles: int, bn: int, recording: bool):
+    """(partial tiles, flags) for a product whose K blocks are dealt out. What a recorded step was given stays as it is for as long
+    as the step may be replayed: a larger scratch is at least twice as large and leaves the smaller one alive, and a recording
+    that finds none large enough gets one of its own, whose flags every replay lowers"""
+    have = _PAIR_SCRATCH.get(device)
+    n, f = tiles * 256 * bn, 8 * tiles
+    if have is not None and have[0].numel() >= n and have[1].numel() >= f:
+        return have
+    if not recording and have is not None:
+        n, f = max(n, 2 * have[0].numel()), max(f, 2 * have[1].numel())
+    made = (torch.empty(n, dtype=torch.float32, device=device), torch.zeros(f, dtype=torch.int32, device=device))
+    if not recording:
+        if have is not None:
+            _PAIR_RETIRED.append(have)
+        _PAIR_SCRATCH[device] = made
+    return made
 
 
 def _prefill_product(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, status: torch.Tensor, swiglu: bool,
@@ -139,13 +162,7 @@ def _prefill_product(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, status
         return
     part = flags = None
     if variant:
-        tiles = -(-m // 256) * -(-n // bn)
-        have = _PAIR_SCRATCH.get(a.device)
-        if have is None or have[0].numel() < tiles * 256 * bn or have[1].numel() < 8 * tiles:
-            have = (torch.empty(tiles * 256 * bn, dtype=torch.float32, device=a.device),
-                    torch.zeros(8 * tiles, dtype=torch.int32, device=a.device))
-            _PAIR_SCRATCH[a.device] = have
-        part, flags = have
+        part, flags = _pair_scratch(a.device, -(-m // 256) * -(-n // bn), bn, _recording(a))
     K.gemm_pair(a, w, out, bn=bn, status=status, swiglu=swiglu, part=part, flags=flags, act=act, act_params=act_params,
                 post=post)
 
@@ -272,7 +289,7 @@ _SK_SCRATCH = {}           # (device, tiles, bn) -> (partial tiles, flags): scra
 def reset_scratch() -> None:
     """lower every flag of the products' scratch (decode gate/up, tiles shared by two pairs of SMs): after a step whose kernels reported an error (a wait
     that ran out can leave a flag raised, which the next step would take for a partial tile that is there)"""
-    for _, flags in list(_SK_SCRATCH.values()) + list(_PAIR_SCRATCH.values()):
+    for _, flags in list(_SK_SCRATCH.values()) + list(_PAIR_SCRATCH.values()) + _PAIR_RETIRED:
         flags.zero_()
 
 
@@ -442,18 +459,19 @@ def _moe_products(ctx, ys, plan, wts, wup, wdown, top, act, T, gated=False, weig
     return planes
 
 
-_ONES = {}
+_ONES = {}                 # device -> ones, and those that more of them took the place of (a recorded step may still read them)
 
 
 def _ones_like(wts: torch.Tensor) -> torch.Tensor:
-    """weights of one for the down product of experts whose weight sits on their input (kept per size and device)"""
-    key = (wts.numel(), wts.device)
-    t = _ONES.get(key)
-    if t is None:
-        if len(_ONES) > 64:
-            _ONES.clear()
-        t = _ONES[key] = torch.ones(wts.numel(), dtype=torch.float32, device=wts.device)
-    return t
+    """weights of one for the down product of experts whose weight sits on their input"""
+    n = wts.numel()
+    kept = _ONES.setdefault(wts.device, [])
+    if kept and kept[-1].numel() >= n:
+        return kept[-1][:n]
+    if _recording(wts):
+        return torch.ones(n, dtype=torch.float32, device=wts.device)       # (written by every replay)
+    kept.append(torch.ones(max(n, 2 * kept[-1].numel() if kept else 0), dtype=torch.float32, device=wts.device))
+    return kept[-1][:n]
 
 
 def moe_experts(ctx, y, idx, wts, wup, wdown, top, act, gated=False, weight_on="output", act_params=None):

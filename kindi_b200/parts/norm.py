@@ -68,7 +68,7 @@ class RMSNorm(Norm):
             return None                     # (a part derived from this one that norms in a way of its own)
         scale = pending.scale
         if scale is not None and scale.dtype != self.weight.dtype:
-            scale = scale.to(self.weight.dtype)
+            return None                     # (the product reads it before its wait: nothing may have written it just now)
         made = L.stream_product(ctx, pending.a, pending.w, x, self.weight, scale)
         return None if made is None else ScaledRows(made[0], made[1], self.eps)
 
