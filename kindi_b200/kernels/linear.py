@@ -12,6 +12,8 @@ import torch
 from . import fast
 from . import lib as K
 
+_base = None            # kindi_b200.parts.base
+
 
 def linear(ctx, a: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype) -> torch.Tensor:
     """a [M, K] @ w [N, K]^T -> [M, N] in out_dtype"""
@@ -41,10 +43,14 @@ def takes_scaled(ctx, w: torch.Tensor, glu: bool = False) -> bool:
 
 
 def branch(ctx, a: torch.Tensor, w: torch.Tensor):
-    """the branch ``a @ w^T``: launched by the norm that adds it, so that a decode-sized step can finish the add and the
-    norm's gains inside the product"""
-    from ..parts.base import LazyBranch
-    return LazyBranch(ctx, a, w)
+    """the branch ``a @ w^T``: in a decode-sized step launched by the norm that adds it, which can then finish the add and its
+    gains inside the product"""
+    global _base
+    if _base is None:
+        from ..parts import base as _base       # (the parts import this module)
+    if a.shape[0] > fast.GEMV_ROWS or not ctx.fast:
+        return _base.Branch(planes(ctx, a, w))
+    return _base.LazyBranch(ctx, a, w)
 
 
 def stream_product(ctx, a: torch.Tensor, w: torch.Tensor, x: torch.Tensor, gain: torch.Tensor, branch_scale):

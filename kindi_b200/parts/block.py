@@ -17,7 +17,7 @@ import torch
 from ..config.registry import part_class, register_part
 from ..config.spec import PartSpec
 from ..kernels import lib as K
-from .base import Block, Branch, StepContext, WeightView
+from .base import Block, Branch, LazyBranch, StepContext, WeightView
 
 _DEFAULT_NAMES = {"norm1": "input_layernorm.", "mixer": "self_attn.", "norm2": "post_attention_layernorm.",
                   "feed_forward": "mlp."}
@@ -96,7 +96,7 @@ class PreNormBlock(Block):
     @staticmethod
     def _norm(ctx: StepContext, norm, reader, x, pending: Optional[Branch]):
         """the rows that ``reader`` reads: undivided, out of the pending branch's own product, where all three allow it"""
-        if pending is not None and reader.takes_scaled_rows(ctx):
+        if isinstance(pending, LazyBranch) and reader.takes_scaled_rows(ctx):
             y = norm.add_norm_scaled(ctx, x, pending)
             if y is not None:
                 return y
